@@ -6,6 +6,7 @@ built raises, and no operation falls back to another implementation.
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
 
 from . import build as _build
@@ -90,6 +91,25 @@ def lib() -> ctypes.CDLL:
         L.ib200_version.restype = i
         _lib = L
     return _lib
+
+
+_host = None
+
+
+def host():
+    """The native host path (csrc/host_ops.cpp), bound to the library ``lib()`` loads."""
+    global _host
+    if _host is None:
+        L = lib()
+        if not os.path.isfile(_build.HOST_PATH):
+            raise ImportError(f"{_build.HOST_PATH} is missing: build it with `python -m inferno_b200.build` (there is no fallback path)")
+        import torch  # noqa: F401  (the module's shared-library dependencies)
+        spec = importlib.util.spec_from_file_location("_host_ops", _build.HOST_PATH)
+        m = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(m)
+        m.bind(L._name, Ib200Error)
+        _host = m
+    return _host
 
 
 def status_string(status: int) -> str:

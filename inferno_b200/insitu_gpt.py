@@ -109,26 +109,8 @@ def run(layers=12, C=768, H=12, vocab=8192, T=1024, B=16, steps=5, warmup=3, see
         for row in evs:
             for e in row:
                 e.record()
-        calls = {"f": 0, "b": 0}
-        orig_f, orig_b = A.attention_forward, A.attention_backward
-
-        def fwd_hook(*a, **kw):
-            i = calls["f"]; calls["f"] += 1
-            A.set_timing_events(evs[i][0], evs[i][1], None, None)
-            try:
-                return orig_f(*a, **kw)
-            finally:
-                A.set_timing_events()          # the hook is per host thread: switch it off where it was switched on
-
-        def bwd_hook(*a, **kw):
-            i = layers - 1 - calls["b"]; calls["b"] += 1
-            A.set_timing_events(None, None, evs[i][2], evs[i][3])
-            try:
-                return orig_b(*a, **kw)       # runs on autograd's worker thread
-            finally:
-                A.set_timing_events()
-
-        A.attention_forward, A.attention_backward = fwd_hook, bwd_hook
+        # forward calls run in layer order, backward calls in reverse
+        A.queue_timing_events([(r[0], r[1]) for r in evs], [(r[2], r[3]) for r in reversed(evs)])
         t0, t1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         try:
             t0.record()
@@ -136,8 +118,7 @@ def run(layers=12, C=768, H=12, vocab=8192, T=1024, B=16, steps=5, warmup=3, see
             t1.record()
             torch.cuda.synchronize()
         finally:
-            A.attention_forward, A.attention_backward = orig_f, orig_b
-            A.set_timing_events()
+            A.queue_timing_events()
         fwd_ms.append(sum(r[0].elapsed_time(r[1]) for r in evs))
         bwd_ms.append(sum(r[2].elapsed_time(r[3]) for r in evs))
         step_ms.append(t0.elapsed_time(t1))

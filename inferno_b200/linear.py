@@ -12,59 +12,22 @@ import torch
 from . import _capi
 
 
-def _check(x: torch.Tensor, name: str):
-    if not x.is_cuda:
-        raise RuntimeError(f"linear: {name} is not on a CUDA device (there is no CPU path)")
-    if x.dtype != torch.bfloat16:
-        raise TypeError(f"linear: {name} must be bfloat16")
-
-
 def linear_forward(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None) -> torch.Tensor:
-    """y = x @ w + bias with x [..., K], w [K, N] (the reference's [in, out] storage), bias [N] fp32."""
-    _check(x, "x"); _check(w, "w")
-    K, N = w.shape
-    x2 = x.reshape(-1, K).contiguous()
-    w = w.contiguous()
-    y = torch.empty((x2.shape[0], N), dtype=torch.bfloat16, device=x.device)
-    b = None if bias is None else bias.to(torch.float32).contiguous()
-    with torch.cuda.device(x.device):
-        rc = _capi.lib().ib200_linear_fwd(x2.data_ptr(), w.data_ptr(), None if b is None else b.data_ptr(), y.data_ptr(),
-                                          x2.shape[0], K, N, torch.cuda.current_stream().cuda_stream)
-    if rc != _capi.OK:
-        raise _capi.Ib200Error(rc, "ib200_linear_fwd")
-    return y.reshape(*x.shape[:-1], N)
+    """y = x @ w + bias with x [..., K], w [K, N] (the reference's [in, out] storage), bias [N]."""
+    return _capi.host().linear_forward(x, w, bias)
 
 
 def linear_backward(x, w, dy, need_dx=True, need_dw=True, need_db=True):
-    K, N = w.shape
-    x2, dy2 = x.reshape(-1, K).contiguous(), dy.reshape(-1, N).contiguous()
-    M = x2.shape[0]
-    dx = torch.empty_like(x2) if need_dx else None
-    dw = torch.empty((K, N), dtype=torch.bfloat16, device=x.device) if need_dw else None
-    db = torch.empty((N,), dtype=torch.float32, device=x.device) if need_db else None
-    ptr = lambda t: None if t is None else t.data_ptr()
-    with torch.cuda.device(x.device):
-        rc = _capi.lib().ib200_linear_bwd(x2.data_ptr(), w.contiguous().data_ptr(), dy2.data_ptr(), ptr(dx), ptr(dw), ptr(db),
-                                          M, K, N, torch.cuda.current_stream().cuda_stream)
-    if rc != _capi.OK:
-        raise _capi.Ib200Error(rc, "ib200_linear_bwd")
-    return (None if dx is None else dx.reshape(x.shape)), dw, db
+    """(dx, dw, db) of ``linear_forward``; db is fp32; what is not needed comes back as None."""
+    return _capi.host().linear_backward(x, w, dy, need_dx, need_dw, need_db)
 
 
-class LinearFunction(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, w, bias):
-        ctx.save_for_backward(x, w)
-        ctx.has_bias = bias is not None
-        ctx.bias_dtype = None if bias is None else bias.dtype
-        return linear_forward(x, w, bias)
+class LinearFunction:
+    """The differentiable projection (backward node in csrc/host_ops.cpp)."""
 
     @staticmethod
-    def backward(ctx, dy):
-        x, w = ctx.saved_tensors
-        dx, dw, db = linear_backward(x, w, dy, ctx.needs_input_grad[0], ctx.needs_input_grad[1],
-                                     ctx.has_bias and ctx.needs_input_grad[2])
-        return dx, dw, (None if db is None else db.to(ctx.bias_dtype))
+    def apply(x, w, bias):
+        return _capi.host().linear(x, w, bias)
 
 
 class Linear(torch.nn.Module):
@@ -77,7 +40,7 @@ class Linear(torch.nn.Module):
         torch.nn.init.normal_(self.weight, 0.0, 0.02)
 
     def forward(self, x):
-        return LinearFunction.apply(x, self.weight, self.bias)
+        return _capi.host().linear(x, self.weight, self.bias)
 
 
 def _time_shape(M: int, K: int, N: int, iters: int = 20):
