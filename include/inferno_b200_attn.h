@@ -126,6 +126,16 @@ int ib200_linear_fwd(const void* x, const void* w, const float* bias, void* y, i
 int ib200_linear_bwd(const void* x, const void* w, const void* dy, void* dx, void* dw, float* db,
                      int M, int K, int N, ib200_stream_t stream);
 
+/* The same two calls with scratch from the caller, and a bias (or bias gradient) of either type (IB200_DTYPE_*).  With a
+ * workspace a product that is cut along K (few output tiles, long K: the weight gradient) is added up in fp32 and rounded
+ * once; without one its parts, at most eight, are rounded to bf16 as they are added.  The workspace need not be
+ * initialised; `ib200_linear_workspace_bytes` gives its size (0: none is used; IB200_PASS_BWD always needs one). */
+size_t ib200_linear_workspace_bytes(int M, int K, int N, int pass);
+int ib200_linear_fwd_ws(const void* x, const void* w, const void* bias, int bias_dtype, void* y, int M, int K, int N,
+                        void* workspace, size_t workspace_bytes, ib200_stream_t stream);
+int ib200_linear_bwd_ws(const void* x, const void* w, const void* dy, void* dx, void* dw, void* db, int db_dtype,
+                        int M, int K, int N, void* workspace, size_t workspace_bytes, ib200_stream_t stream);
+
 /* Capacity in bytes of the scratch buffer that is compiled into the library for
  * ib200_attn_bwd_static (one copy lives in the memory of every GPU that loads the library,
  * from load until the process exits). */
@@ -165,7 +175,7 @@ int ib200_attn_bwd_static(const void* q, const void* k, const void* v, const voi
 int ib200_attn_check(const void* workspace, ib200_stream_t stream, int* device_code);
 
 /* The same check for the calls that have no caller workspace: ib200_attn_bwd_static and the
- * projection entry points (ib200_gemm_bf16, ib200_linear_fwd, ib200_linear_bwd) record an expired
+ * projection entry points (ib200_gemm_bf16, ib200_linear_*) record an expired
  * wait in the header of the library's built-in buffer on the current device; this reads and clears
  * it after synchronising `stream`.  Same return values as ib200_attn_check.  Replaces the same
  * check_cuda() convention (src/inferno/cuda/cudaops.h:198-210). */

@@ -22,7 +22,7 @@ EXPORTS = (
     "ib200_attn_workspace_bytes", "ib200_attn_fwd", "ib200_attn_bwd", "ib200_attn_check",
     "ib200_status_string", "ib200_last_cuda_error", "ib200_version", "ib200_attn_set_timing_events", "ib200_attn_bwd_static", "ib200_attn_fwd_strided", "ib200_attn_bwd_strided", "ib200_gemm_bf16", "ib200_linear_fwd", "ib200_linear_bwd",
     "ib200_cast_f32_to_bf16", "ib200_cast_bf16_to_f32", "ib200_attn_item_order", "ib200_attn_check_static",
-    "ib200_selftest_wait_expiry",
+    "ib200_selftest_wait_expiry", "ib200_linear_workspace_bytes", "ib200_linear_fwd_ws", "ib200_linear_bwd_ws",
 )
 
 

@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 #include <math.h>
 
+#include <algorithm>
 #include <atomic>
 
 #include "attn_aux.cuh"
@@ -75,33 +76,23 @@ bool make_tmap(CUtensorMap* m, const void* base, bool f32, int D, int T, const R
     return r == CUDA_SUCCESS;
 }
 
-// Tensor map over a row-major bf16 matrix [rows, cols]; box = [box_rows x 64 columns], 128B swizzle.
-bool make_tmap_2d(CUtensorMap* m, const void* base, long rows, long cols, int box_rows) {
+// Tensor map over a row-major matrix [rows, cols] of bf16 or fp32; box = [box_rows x 128 bytes], 128B swizzle.
+bool make_tmap_2d(CUtensorMap* m, const void* base, long rows, long cols, int box_rows, bool f32 = false) {
     EncodeTiledFn enc = encode_fn();
     if (!enc) return false;
+    const cuuint64_t es = f32 ? 4 : 2;
     cuuint64_t dims[3] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows), 1};
-    cuuint64_t strides[2] = {static_cast<cuuint64_t>(cols) * 2, static_cast<cuuint64_t>(rows) * static_cast<cuuint64_t>(cols) * 2};
-    cuuint32_t box[3] = {64, static_cast<cuuint32_t>(box_rows), 1};
+    cuuint64_t strides[2] = {static_cast<cuuint64_t>(cols) * es, static_cast<cuuint64_t>(rows) * static_cast<cuuint64_t>(cols) * es};
+    cuuint32_t box[3] = {static_cast<cuuint32_t>(128 / es), static_cast<cuuint32_t>(box_rows), 1};
     cuuint32_t estr[3] = {1, 1, 1};
-    return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    return enc(m, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 inline size_t round_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 constexpr size_t kHeaderBytes = 256;
-
-// Workspace header: word 0 = device status (sticky: the first expired wait stays recorded until ib200_attn_check
-// has read it), word 1 = draw counter of the persistent kernels (zero at every launch), word 3 = "status word is
-// valid" mark.  A workspace arrives uninitialised, so the mark decides whether word 0 is a status or garbage.
-__global__ void prepare_header_kernel(int* hdr) {
-    if (threadIdx.x == 0) prepare_header(hdr);
-}
-int prepare_header(void* ws, cudaStream_t stream) {
-    prepare_header_kernel<<<1, 32, 0, stream>>>(static_cast<int*>(ws));
-    return launch_status();
-}
 
 struct Problem {
     long BH, N;        // heads, elements per tensor
@@ -127,12 +118,52 @@ size_t bwd_ws_bytes(long N, long BH, int T, bool f32) {
            (f32 ? 8 * round_up(N * 2, 256) : 0);
 }
 
-int device_ok() {
+constexpr int kMaxDevices = 64;
+// What a launch needs to know of the current device, asked of the driver once per device.
+struct DeviceInfo {
+    std::atomic<int> state{0};      // 0: not asked, 1: no sm_100 device, 2: usable
+    int sms = 0, index = 0;
+};
+// Also makes the device's primary context current on this host thread (a framework's worker thread may never have touched
+// CUDA), which the tensor-map encoder needs.
+const DeviceInfo* device_info() {
+    static DeviceInfo table[kMaxDevices];
+    thread_local int entered = -1;
     int dev = 0;
-    if (!cuda_ok(cudaGetDevice(&dev))) return IB200_ERR_NO_DEVICE;
-    int major = 0;
-    if (!cuda_ok(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev))) return IB200_ERR_NO_DEVICE;
-    return major == 10 ? IB200_OK : IB200_ERR_NO_DEVICE;
+    if (!cuda_ok(cudaGetDevice(&dev)) || dev < 0 || dev >= kMaxDevices) return nullptr;
+    DeviceInfo& d = table[dev];
+    int state = d.state.load(std::memory_order_acquire);
+    if (state == 0) {
+        // host threads that race here ask the same question and store the same answer
+        int major = 0, sms = 0;
+        if (!cuda_ok(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev)) ||
+            !cuda_ok(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)))
+            return nullptr;
+        d.sms = sms;
+        d.index = dev;
+        state = major == 10 ? 2 : 1;
+        d.state.store(state, std::memory_order_release);
+    }
+    if (state != 2) return nullptr;
+    if (entered != dev) {
+        if (!cuda_ok(cudaFree(nullptr))) return nullptr;
+        entered = dev;
+    }
+    return &d;
+}
+int device_ok() { return device_info() ? IB200_OK : IB200_ERR_NO_DEVICE; }
+
+// Dynamic shared memory beyond 48 KB has to be allowed once per kernel and device.
+template <auto KERNEL>
+bool allow_smem(int bytes) {
+    static std::atomic<unsigned long long> done{0};
+    const DeviceInfo* d = device_info();
+    if (!d) return false;
+    const unsigned long long bit = 1ull << d->index;
+    if (done.load(std::memory_order_relaxed) & bit) return true;
+    if (!cuda_ok(cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes))) return false;
+    done.fetch_or(bit, std::memory_order_relaxed);
+    return true;
 }
 
 // Number of head groups of a persistent kernel's item list (see locate_item).  The CTAs draw items in list order, so at
@@ -168,8 +199,8 @@ int launch_fwd_persist(const void* q, const void* q_lo, const void* k, const voi
     } else {
         tql = tq; tkl = tk; tvl = tv;
     }
-    if (!cuda_ok(cudaFuncSetAttribute(attn_fwd_persist_kernel<TR>, cudaFuncAttributeMaxDynamicSharedMemorySize, TR::SMEM_BYTES)))
-        return IB200_ERR_CUDA;
+    const DeviceInfo* dev = device_info();
+    if (!dev || !allow_smem<attn_fwd_persist_kernel<TR>>(TR::SMEM_BYTES)) return IB200_ERR_CUDA;
     FwdPersistParams pp;
     pp.p.lse = lse;
     pp.p.status = status;
@@ -182,17 +213,13 @@ int launch_fwd_persist(const void* q, const void* q_lo, const void* k, const voi
     const long items = static_cast<long>(pp.pairs_per_head) * BH;
     if (items > 0x7fffffffL) return IB200_ERR_UNSUPPORTED;
     pp.n_items = static_cast<int>(items);
-    int dev = 0, sms = 148;
-    if (cuda_ok(cudaGetDevice(&dev))) (void)cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int grid = static_cast<int>(items < sms ? items : sms);
+    const int sms = dev->sms;
     pp.n_groups = persist_head_groups(sms, pp.pairs_per_head, BH, static_cast<size_t>(T) * D * (SPLIT ? 8 : 4) /*K, V*/);
-    pp.next_item = status + 1;              // second word of the workspace header, zeroed before every launch
     IB200_SET_BOUNDS(D, T, lq.H, static_cast<int>(BH / lq.H), static_cast<int>(BH), 0, TR::TM_COLS, status, stream);
     record_timing_event(0, stream);
-    attn_fwd_persist_kernel<TR><<<grid, TR::THREADS, TR::SMEM_BYTES, stream>>>(tq, tql, tk, tkl, tv, tvl, to, pp);
-    const bool launched = cuda_ok(cudaGetLastError());
+    const int rc = launch_pdl<attn_fwd_persist_kernel<TR>>(pp.n_items, TR::THREADS, TR::SMEM_BYTES, stream, tq, tql, tk, tkl, tv, tvl, to, pp);
     record_timing_event(1, stream);
-    return launched ? IB200_OK : IB200_ERR_CUDA;
+    return rc;
 }
 
 // Persistent CTAs walking (head, key tile) items, longest walks first.  SPLIT (fp32 I/O): every operand is given as dense
@@ -223,8 +250,8 @@ int launch_bwd_persist(const void* const q[2], const void* const k[2], const voi
                 CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return IB200_ERR_CUDA;
     }
-    if (!cuda_ok(cudaFuncSetAttribute(attn_bwd_persist_kernel<TR>, cudaFuncAttributeMaxDynamicSharedMemorySize, TR::SMEM_BYTES)))
-        return IB200_ERR_CUDA;
+    const DeviceInfo* dev = device_info();
+    if (!dev || !allow_smem<attn_bwd_persist_kernel<TR>>(TR::SMEM_BYTES)) return IB200_ERR_CUDA;
     BwdParams prm;
     prm.nlse2 = nlse2;
     prm.ndelta = ndelta;
@@ -239,19 +266,15 @@ int launch_bwd_persist(const void* const q[2], const void* const k[2], const voi
     prm.dq_scale = dq_scale;
     const long items = static_cast<long>((T + TR::BKV - 1) / TR::BKV) * BH;
     if (items > 0x7fffffffL) return IB200_ERR_UNSUPPORTED;
-    int dev = 0, sms = 148;
-    if (cuda_ok(cudaGetDevice(&dev))) (void)cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int grid = static_cast<int>(items < sms ? items : sms);
+    const int sms = dev->sms;
     const int n_groups = persist_head_groups(sms, (T + TR::BKV - 1) / TR::BKV, BH,
                                              static_cast<size_t>(T) * TR::D * (TR::SPLIT ? 12 : 8) /*Q, dO (hi + lo), fp32 dQ*/);
     IB200_SET_BOUNDS(TR::D, T, lq.H, static_cast<int>(BH / lq.H), static_cast<int>(BH), 0, TR::TM_COLS, status, stream);
     record_timing_event(2, stream);
-    attn_bwd_persist_kernel<TR><<<grid, TR::THREADS, TR::SMEM_BYTES, stream>>>(tq[0], tq[1], tk[0], tk[1], tv[0], tv[1], tdo[0], tdo[1], tdk, tdv, tdq, prm,
-                                                                               static_cast<int>(items), n_groups,
-                                                                               status + 1 /*draw counter: header word zeroed before every launch*/);
-    const bool launched = cuda_ok(cudaGetLastError());
+    const int rc = launch_pdl<attn_bwd_persist_kernel<TR>>(static_cast<int>(items), TR::THREADS, TR::SMEM_BYTES, stream, tq[0], tq[1], tk[0], tk[1], tv[0], tv[1],
+                                                           tdo[0], tdo[1], tdk, tdv, tdq, prm, static_cast<int>(items), n_groups);
     record_timing_event(3, stream);
-    return launched ? IB200_OK : IB200_ERR_CUDA;
+    return rc;
 }
 
 struct BwdLayouts {
@@ -281,7 +304,6 @@ int launch_bwd_typed(const void* q, const void* k, const void* v, const void* o,
     job.o = o; job.dO = dO; job.lse = lse; job.ndelta = ndelta; job.nlse2 = nlse2;
     job.lo = L.o; job.ldo = L.dO;
     job.dq_acc = reinterpret_cast<float4*>(dq_acc);
-    job.header = status;
     const void* qp[2] = {q, q}; const void* kp[2] = {k, k}; const void* vp[2] = {v, v}; const void* dop[2] = {dO, dO};
     RowLayout lq = L.q, lk = L.k, lv = L.v, ldo = L.dO;
     if (F32) {
@@ -334,7 +356,6 @@ int resolve_layout(const ib200_layout* in, int H, int T, int D, bool f32, RowLay
 // the launch path receives.
 static __device__ __align__(256) unsigned char g_static_scratch[IB200_STATIC_SCRATCH_BYTES];
 
-constexpr int kMaxDevices = 64;
 // Filled on first use per device.  Two host threads that race on the first call both look the address up and both
 // store the same value, so a relaxed atomic is all the cache needs.
 std::atomic<void*> g_static_scratch_addr[kMaxDevices];
@@ -380,56 +401,160 @@ bool header_is_builtin(const void* header) {
     return false;
 }
 
-template <bool A_MN, bool B_MN>
-int launch_gemm(const void* a, const void* b, void* c, const float* bias, int M, int N, int K, cudaStream_t stream) {
+// ---- projections -------------------------------------------------------------------
+struct GemmDesc {
+    const void *a, *b;
+    void* c;
+    int M, N, K, a_mn, b_mn;
+    int tiles() const { return ((M + GemmTraits::BM - 1) / GemmTraits::BM) * ((N + GemmTraits::BN - 1) / GemmTraits::BN); }
+    int k_slices() const { return (K + GemmTraits::BK - 1) / GemmTraits::BK; }
+};
+
+bool gemm_set_task(GemmParams& p, GemmMaps& m, int i, const GemmDesc& d) {
     using TR = GemmTraits;
-    // a runtime call first: it makes the primary context current on this host thread (a framework's worker
-    // thread may never have touched CUDA), which the driver's tensor-map encoder needs
-    if (!cuda_ok(cudaFuncSetAttribute(gemm_bf16_kernel<A_MN, B_MN>, cudaFuncAttributeMaxDynamicSharedMemorySize, TR::SMEM_BYTES)))
-        return IB200_ERR_CUDA;
-    CUtensorMap ta, tb, tc;
-    // A: [M,K] (box 128 rows) or stored [K,M] (box 64 k-rows); B: stored [K,N] (box 64 k-rows) or [N,K] (box 256 rows)
-    const bool ok = (A_MN ? make_tmap_2d(&ta, a, K, M, 64) : make_tmap_2d(&ta, a, M, K, 128)) &&
-                    (B_MN ? make_tmap_2d(&tb, b, K, N, 64) : make_tmap_2d(&tb, b, N, K, 256)) && make_tmap_2d(&tc, c, M, N, 128);
-    if (!ok) return IB200_ERR_CUDA;
-    int dev = 0, sms = 148;
-    if (cuda_ok(cudaGetDevice(&dev))) (void)cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const long tiles = static_cast<long>((M + TR::BM - 1) / TR::BM) * ((N + TR::BN - 1) / TR::BN);
-    // Split-K when the tiles would leave more than half of the SMs idle and K is long enough to cut: as many slabs as
-    // fit in one wave, each at least eight 64-wide k-slices.  The slabs add into C, so C is zeroed first.
-    const int k_slices = (K + TR::BK - 1) / TR::BK;
-    int splits = 1;
-    if (tiles * 2 <= sms) {
-        splits = static_cast<int>(sms / tiles);
-        if (splits > 8) splits = 8;
-        while (splits > 1 && k_slices / splits < 8) --splits;
-    }
-    if (splits > 1 && !cuda_ok(cudaMemsetAsync(c, 0, static_cast<size_t>(M) * N * 2, stream))) return IB200_ERR_CUDA;
-    GemmParams prm;
-    prm.bias = bias;
-    prm.M = M; prm.N = N; prm.K = K;
-    prm.splits = splits;
-    // an expired wait is recorded in the status word of the library's built-in buffer (read by ib200_attn_check_static)
-    void* builtin = nullptr;
-    prm.status = static_scratch(&builtin) == IB200_OK ? static_cast<int*>(builtin) : nullptr;
-    const long units = tiles * splits;
-    const int grid = static_cast<int>(units < sms ? units : sms);       // persistent: one CTA per SM
-    IB200_SET_BOUNDS(0, 0, 0, 0, 0, 1, TR::TM_COLS, prm.status, stream);
-    gemm_bf16_kernel<A_MN, B_MN><<<grid, TR::THREADS, TR::SMEM_BYTES, stream>>>(ta, tb, tc, prm);
-    return cuda_ok(cudaGetLastError()) ? IB200_OK : IB200_ERR_CUDA;
+    p.t[i] = GemmTask{d.M, d.N, (d.M + TR::BM - 1) / TR::BM, d.tiles(), d.k_slices(), d.a_mn, d.b_mn};
+    // A: [M, K] (box 128 rows) or stored [K, M] (box 64 k-rows); B: stored [K, N] (box 64 k-rows) or [N, K] (box 128 rows)
+    return (d.a_mn ? make_tmap_2d(&m.a[i], d.a, d.K, d.M, TR::BK) : make_tmap_2d(&m.a[i], d.a, d.M, d.K, TR::CM)) &&
+           (d.b_mn ? make_tmap_2d(&m.b[i], d.b, d.K, d.N, TR::BK) : make_tmap_2d(&m.b[i], d.b, d.N, d.K, TR::CN)) &&
+           make_tmap_2d(&m.c[i], d.c, d.M, d.N, 32);
 }
 
-int gemm_dispatch(const void* a, const void* b, void* c, const float* bias, int M, int N, int K, int a_t, int b_t, cudaStream_t stream) {
-    if (!a || !b || !c) return IB200_ERR_INVALID_ARGUMENT;
-    if (M <= 0 || N <= 0 || K <= 0 || (a_t != 0 && a_t != 1) || (b_t != 0 && b_t != 1)) return IB200_ERR_INVALID_ARGUMENT;
-    if (M % 8 || N % 8 || K % 8) return IB200_ERR_UNSUPPORTED;
-    if (!aligned16(a) || !aligned16(b) || !aligned16(c) || (bias && !aligned16(bias))) return IB200_ERR_MISALIGNED;
-    int rc = device_ok();
+// A product is cut along K when its tiles would leave more than half of the CTA pairs idle and K is at least two parts long.
+constexpr int kMinPartSlices = 8;      // shorter parts spend more on adding up than on multiplying
+bool gemm_wants_split(const GemmDesc& d, int pairs) { return d.tiles() * 2 <= pairs && d.k_slices() >= 2 * kMinPartSlices; }
+// Next to other tiles (dX) a product with no more tiles than two rounds is cut as well: its slices then even out the load.
+bool gemm_wants_split_beside(const GemmDesc& d, int pairs) { return d.tiles() <= 2 * pairs && d.k_slices() >= 2 * kMinPartSlices; }
+
+// One launch: `whole` cut into whole tiles (may be null), `other` cut into whole tiles or, with split != kPartWhole, along K.
+int launch_gemms(const GemmDesc* whole, const GemmDesc* other, int split, float* acc, const void* bias, int bias_bf16, cudaStream_t stream) {
+    using TR = GemmTraits;
+    const DeviceInfo* dev = device_info();
+    if (!dev || !allow_smem<gemm_bf16_kernel>(TR::SMEM_BYTES)) return IB200_ERR_CUDA;
+    const int max_pairs = dev->sms / 2;
+    GemmMaps maps;
+    GemmParams p{};
+    if ((whole && !gemm_set_task(p, maps, 0, *whole)) || (other && !gemm_set_task(p, maps, 1, *other))) return IB200_ERR_CUDA;
+    if (!whole) { maps.a[0] = maps.a[1]; maps.b[0] = maps.b[1]; maps.c[0] = maps.c[1]; }
+    if (!other) { maps.a[1] = maps.a[0]; maps.b[1] = maps.b[0]; maps.c[1] = maps.c[0]; }
+    maps.sum = maps.c[1];
+    if (split == kPartReduceF32 && !make_tmap_2d(&maps.sum, acc, other->M, other->N, 32, true)) return IB200_ERR_CUDA;
+    p.split = split;
+    p.bias = bias;
+    p.bias_bf16 = bias_bf16;
+    long tiles = p.t[0].tiles;
+    int pairs;
+    if (split == kPartWhole) {
+        tiles += p.t[1].tiles;
+        pairs = static_cast<int>(tiles < max_pairs ? tiles : max_pairs);
+    } else {
+        // every pair shall end up with the same number of k-slices: `heavy` pairs own one whole tile (k0 slices) more than the rest
+        const long long W = static_cast<long long>(p.t[1].tiles) * p.t[1].k_slices, k0 = whole ? p.t[0].k_slices : 0;
+        // partial tiles that are rounded to bf16 as they are added: at most eight per tile
+        const long long min_part = split == kPartReduceBf16 ? std::max<long long>(kMinPartSlices, (p.t[1].k_slices + 6) / 7) : kMinPartSlices;
+        const long long most = std::max(1LL, W / min_part);
+        if (p.t[0].tiles < max_pairs) {
+            p.heavy = p.t[0].tiles;
+            pairs = p.heavy + static_cast<int>(std::min<long long>(max_pairs - p.heavy, most));
+        } else {
+            p.heavy = p.t[0].tiles % max_pairs;
+            pairs = max_pairs;
+        }
+        const long long light = pairs - p.heavy;
+        p.w_heavy = std::max(0LL, W - light * k0);
+        p.w_light = p.w_heavy > 0 ? p.w_heavy + pairs * k0 : 1;
+        p.w_total = p.heavy * p.w_heavy + light * p.w_light;
+    }
+    // an expired wait is recorded in the status word of the library's built-in buffer (read by ib200_attn_check_static)
+    void* builtin = nullptr;
+    p.status = static_scratch(&builtin) == IB200_OK ? static_cast<int*>(builtin) : nullptr;
+    IB200_SET_BOUNDS(0, 0, 0, 0, 0, 1, TR::TM_COLS, p.status, stream);
+    return launch_pdl<gemm_bf16_kernel>(2 * pairs, TR::THREADS, TR::SMEM_BYTES, stream, maps, p);
+}
+
+int gemm_check(const GemmDesc& d) {
+    if (!d.a || !d.b || !d.c) return IB200_ERR_INVALID_ARGUMENT;
+    if (d.M <= 0 || d.N <= 0 || d.K <= 0 || (d.a_mn != 0 && d.a_mn != 1) || (d.b_mn != 0 && d.b_mn != 1)) return IB200_ERR_INVALID_ARGUMENT;
+    if (d.M % 8 || d.N % 8 || d.K % 8) return IB200_ERR_UNSUPPORTED;
+    if (!aligned16(d.a) || !aligned16(d.b) || !aligned16(d.c)) return IB200_ERR_MISALIGNED;
+    return device_ok();
+}
+
+int launch_linear_finish(const float* acc, void* out, long n, const float* part, int slabs, int N, void* db, int db_bf16, cudaStream_t stream) {
+    const long n8 = n / 8;
+    const int db_blocks = db ? (N + kFinishCols - 1) / kFinishCols : 0;
+    long blocks = acc ? std::min<long>((n8 + 255) / 256, 148 * 8) : 0;
+    if (blocks + db_blocks == 0) return IB200_OK;
+    return launch_pdl<linear_finish_kernel>(static_cast<int>(blocks) + db_blocks, 256, 0, stream, reinterpret_cast<const float4*>(acc), static_cast<uint4*>(out), n8,
+                                            part, slabs, N, db, db_bf16, db_blocks);
+}
+
+// One product.  With a workspace of at least M * N floats a split product is added up in fp32.
+int gemm_single(const GemmDesc& d, const void* bias, int bias_bf16, void* ws, size_t ws_bytes, cudaStream_t stream) {
+    int rc = gemm_check(d);
     if (rc != IB200_OK) return rc;
-    if (!a_t && !b_t) return launch_gemm<false, true>(a, b, c, bias, M, N, K, stream);
-    if (!a_t && b_t) return launch_gemm<false, false>(a, b, c, bias, M, N, K, stream);
-    if (a_t && !b_t) return launch_gemm<true, true>(a, b, c, bias, M, N, K, stream);
-    return launch_gemm<true, false>(a, b, c, bias, M, N, K, stream);
+    if (bias && !aligned16(bias)) return IB200_ERR_MISALIGNED;
+    const DeviceInfo* dev = device_info();
+    if (!dev) return IB200_ERR_CUDA;
+    if (!gemm_wants_split(d, dev->sms / 2)) return launch_gemms(&d, nullptr, kPartWhole, nullptr, bias, bias_bf16, stream);
+    const size_t n = static_cast<size_t>(d.M) * d.N;
+    if (!ws || ws_bytes < n * 4) {
+        if (!cuda_ok(cudaMemsetAsync(d.c, 0, n * 2, stream))) return IB200_ERR_CUDA;
+        return launch_gemms(nullptr, &d, kPartReduceBf16, nullptr, bias, bias_bf16, stream);
+    }
+    if (!cuda_ok(cudaMemsetAsync(ws, 0, n * 4, stream))) return IB200_ERR_CUDA;
+    if ((rc = launch_gemms(nullptr, &d, kPartReduceF32, static_cast<float*>(ws), bias, bias_bf16, stream))) return rc;
+    return launch_linear_finish(static_cast<const float*>(ws), d.c, static_cast<long>(n), nullptr, 0, 0, nullptr, 0, stream);
+}
+
+// Row slabs of the column sums: enough blocks for the chip, and few enough partial sums to add up afterwards.
+int colsum_slabs(int M, int N) {
+    const int gx = (N + kColsumCols - 1) / kColsumCols;
+    const int by_blocks = (4 * 148 + gx - 1) / gx, by_rows = (M + 63) / 64;
+    return std::max(1, std::min(std::min(by_blocks, by_rows), kMaxColsumSlabs));
+}
+size_t linear_bwd_ws_bytes(int K, int N) { return round_up(static_cast<size_t>(K) * N * 4, 256) + static_cast<size_t>(kMaxColsumSlabs) * N * 4; }
+
+int linear_bwd_core(const void* x, const void* w, const void* dy, void* dx, void* dw, void* db, int db_bf16, int M, int K, int N, void* ws, size_t ws_bytes,
+                    cudaStream_t stream) {
+    if (!x || !w || !dy) return IB200_ERR_INVALID_ARGUMENT;
+    // dx[M,K] = dy[M,N] w^T: w is stored [K, N], i.e. the "B" of this product stored [N_out = K rows, contraction N contiguous]
+    const GemmDesc gx{dy, w, dx, M, K, N, 0, 0};
+    // dw[K,N] = x^T dy: x is stored [M, K], i.e. the "A" of this product stored [contraction M rows, K contiguous]
+    const GemmDesc gw{x, dy, dw, K, N, M, 1, 1};
+    int rc;
+    if (dx && (rc = gemm_check(gx))) return rc;
+    if (dw && (rc = gemm_check(gw))) return rc;
+    if (db && (M <= 0 || N <= 0)) return IB200_ERR_INVALID_ARGUMENT;
+    if (db && N % 8) return IB200_ERR_UNSUPPORTED;
+    if (!aligned16(dy)) return IB200_ERR_MISALIGNED;
+    const bool have_ws = ws && aligned16(ws) && ws_bytes >= linear_bwd_ws_bytes(K, N);
+    if (db && db_bf16 && !have_ws) return IB200_ERR_WORKSPACE;
+    const DeviceInfo* dev = device_info();
+    if (!dev) return IB200_ERR_CUDA;
+    const int pairs = dev->sms / 2;
+    const bool split = dw && have_ws && (dx ? gemm_wants_split_beside(gw, pairs) : gemm_wants_split(gw, pairs));
+    float* acc = split ? static_cast<float*>(ws) : nullptr;
+    float* part = nullptr;
+    const int slabs = colsum_slabs(M, N);
+    if (db) {
+        part = have_ws ? reinterpret_cast<float*>(static_cast<uint8_t*>(ws) + round_up(static_cast<size_t>(K) * N * 4, 256)) : static_cast<float*>(db);
+        if (!have_ws && !cuda_ok(cudaMemsetAsync(db, 0, static_cast<size_t>(N) * 4, stream))) return IB200_ERR_CUDA;
+    }
+    if (db || split) {
+        const int rows = (M + slabs - 1) / slabs;
+        const dim3 grid((N + kColsumCols - 1) / kColsumCols, db ? slabs : 64);
+        if ((rc = launch_pdl<linear_prep_kernel>(grid, 256, 0, stream, static_cast<const __nv_bfloat16*>(dy), part, M, N, rows, have_ws ? 0 : 1,
+                                                 reinterpret_cast<float4*>(acc), split ? static_cast<long>(K) * N / 4 : 0)))
+            return rc;
+    }
+    if (have_ws && dx && dw) {
+        if ((rc = launch_gemms(&gx, &gw, split ? kPartReduceF32 : kPartWhole, acc, nullptr, 0, stream))) return rc;
+    } else {
+        if (dx && (rc = gemm_single(gx, nullptr, 0, nullptr, 0, stream))) return rc;
+        if (dw && split && (rc = launch_gemms(nullptr, &gw, kPartReduceF32, acc, nullptr, 0, stream))) return rc;
+        if (dw && !split && (rc = gemm_single(gw, nullptr, 0, nullptr, 0, stream))) return rc;
+    }
+    return launch_linear_finish(acc, dw, static_cast<long>(K) * N, part, slabs, N, have_ws ? db : nullptr, db_bf16, stream);
 }
 
 int fwd_core(const void* q, const void* k, const void* v, void* o, float* lse, const ib200_layout* lq_, const ib200_layout* lk_,
@@ -453,7 +578,6 @@ int fwd_core(const void* q, const void* k, const void* v, void* o, float* lse, c
 
     uint8_t* ws = static_cast<uint8_t*>(workspace);
     int* status = reinterpret_cast<int*>(ws);
-    if (!f32 && (rc = prepare_header(ws, stream))) return rc;      // fp32 I/O: the split pre-pass prepares the header
     if (f32) {
         // fp32 operands are carried as dense (hi, lo) bf16 pairs
         const size_t slab = round_up(N * 2, 256);
@@ -470,7 +594,7 @@ int fwd_core(const void* q, const void* k, const void* v, void* o, float* lse, c
             job.lin[i] = *lsrc[i];
         }
         job.in[3] = nullptr; job.hi[3] = job.lo[3] = nullptr; job.lin[3] = lq;
-        rc = launch_split_bf16(job, 3, status, BH, T, D, stream);
+        rc = launch_split_bf16(job, 3, BH, T, D, stream);
         if (rc) return rc;
         const RowLayout dl = dense_layout(H, T, D);
         return launch_fwd_persist<64, true>(part[0], part[1], part[2], part[3], part[4], part[5], o, dl, dl, dl, lo, lse, status, BH, T,
@@ -511,7 +635,7 @@ int bwd_core(const void* q, const void* k, const void* v, const void* o, const v
         if (rc != IB200_OK) return rc;
         ws = static_cast<uint8_t*>(scratch);
     }
-    // launch_bwd_all clears the header and the dQ accumulator on `stream` and rewrites every other part of the
+    // launch_bwd_all clears the dQ accumulator on `stream` and rewrites every other part of the
     // scratch it reads, so stale contents of an earlier call (static scratch is shared) are never consumed
     return launch_bwd_all(q, k, v, o, dO, lse, dq, dk, dv, L, BH, T, D, scale, causal, f32, ws, stream);
 }
@@ -652,35 +776,40 @@ int ib200_attn_bwd_static(const void* q, const void* k, const void* v, const voi
 
 int ib200_gemm_bf16(const void* a, const void* b, void* c, const float* bias, int M, int N, int K, int a_transposed,
                     int b_transposed, ib200_stream_t stream) {
-    return gemm_dispatch(a, b, c, bias, M, N, K, a_transposed, b_transposed, reinterpret_cast<cudaStream_t>(stream));
+    return gemm_single(GemmDesc{a, b, c, M, N, K, a_transposed, b_transposed == 0 ? 1 : b_transposed == 1 ? 0 : -1}, bias, 0, nullptr, 0,
+                       reinterpret_cast<cudaStream_t>(stream));
 }
 
 int ib200_linear_fwd(const void* x, const void* w, const float* bias, void* y, int M, int K, int N, ib200_stream_t stream) {
-    return gemm_dispatch(x, w, y, bias, M, N, K, 0, 0, reinterpret_cast<cudaStream_t>(stream));
+    return gemm_single(GemmDesc{x, w, y, M, N, K, 0, 1}, bias, 0, nullptr, 0, reinterpret_cast<cudaStream_t>(stream));
 }
 
 int ib200_linear_bwd(const void* x, const void* w, const void* dy, void* dx, void* dw, float* db, int M, int K, int N,
-                     ib200_stream_t stream_) {
-    cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
-    if (!x || !w || !dy) return IB200_ERR_INVALID_ARGUMENT;
-    int rc = IB200_OK;
-    // dx[M,K] = dy[M,N] w^T: w is stored [K, N], i.e. the "B" of this product stored [N_out = K rows, contraction N contiguous]
-    if (dx && (rc = gemm_dispatch(dy, w, dx, nullptr, M, K, N, 0, 1, stream))) return rc;
-    // dw[K,N] = x^T dy: x is stored [M, K], i.e. the "A" of this product stored [contraction M rows, K contiguous]
-    if (dw && (rc = gemm_dispatch(x, dy, dw, nullptr, K, N, M, 1, 0, stream))) return rc;
-    if (db) {
-        if (N % 8) return IB200_ERR_UNSUPPORTED;
-        // row slabs so that the grid covers the SMs a few times over; the slabs meet in fp32 atomics on a zeroed db
-        int slabs = (4 * 148 + (N + 63) / 64 - 1) / ((N + 63) / 64);
-        if (slabs > (M + 255) / 256) slabs = (M + 255) / 256;
-        if (slabs < 1) slabs = 1;
-        const int rows_per_block = ((M + slabs - 1) / slabs + 7) / 8 * 8;
-        if (!cuda_ok(cudaMemsetAsync(db, 0, static_cast<size_t>(N) * 4, stream))) return IB200_ERR_CUDA;
-        colsum_bf16_kernel<<<dim3((N + 63) / 64, (M + rows_per_block - 1) / rows_per_block), 256, 0, stream>>>(
-            static_cast<const __nv_bfloat16*>(dy), db, M, N, rows_per_block);
-        if (!cuda_ok(cudaGetLastError())) return IB200_ERR_CUDA;
-    }
-    return IB200_OK;
+                     ib200_stream_t stream) {
+    return linear_bwd_core(x, w, dy, dx, dw, db, 0, M, K, N, nullptr, 0, reinterpret_cast<cudaStream_t>(stream));
+}
+
+size_t ib200_linear_workspace_bytes(int M, int K, int N, int pass) {
+    if (M <= 0 || K <= 0 || N <= 0) return 0;
+    if (pass == IB200_PASS_BWD) return linear_bwd_ws_bytes(K, N);
+    const GemmDesc d{nullptr, nullptr, nullptr, M, N, K, 0, 1};
+    const DeviceInfo* dev = device_info();
+    return dev && gemm_wants_split(d, dev->sms / 2) ? static_cast<size_t>(M) * N * 4 : 0;
+}
+
+int ib200_linear_fwd_ws(const void* x, const void* w, const void* bias, int bias_dtype, void* y, int M, int K, int N, void* workspace,
+                        size_t workspace_bytes, ib200_stream_t stream) {
+    if (bias_dtype != IB200_DTYPE_F32 && bias_dtype != IB200_DTYPE_BF16) return IB200_ERR_INVALID_ARGUMENT;
+    if (workspace && !aligned16(workspace)) return IB200_ERR_WORKSPACE;
+    return gemm_single(GemmDesc{x, w, y, M, N, K, 0, 1}, bias, bias_dtype == IB200_DTYPE_BF16, workspace, workspace_bytes,
+                       reinterpret_cast<cudaStream_t>(stream));
+}
+
+int ib200_linear_bwd_ws(const void* x, const void* w, const void* dy, void* dx, void* dw, void* db, int db_dtype, int M, int K, int N, void* workspace,
+                        size_t workspace_bytes, ib200_stream_t stream) {
+    if (db_dtype != IB200_DTYPE_F32 && db_dtype != IB200_DTYPE_BF16) return IB200_ERR_INVALID_ARGUMENT;
+    if (!workspace || !aligned16(workspace) || (M > 0 && K > 0 && N > 0 && workspace_bytes < linear_bwd_ws_bytes(K, N))) return IB200_ERR_WORKSPACE;
+    return linear_bwd_core(x, w, dy, dx, dw, db, db_dtype == IB200_DTYPE_BF16, M, K, N, workspace, workspace_bytes, reinterpret_cast<cudaStream_t>(stream));
 }
 
 static int read_and_clear_status(void* header, cudaStream_t stream, int* device_code) {
@@ -706,7 +835,6 @@ int ib200_selftest_wait_expiry(void* workspace, size_t workspace_bytes, unsigned
     if (limit_us == 0 || limit_us > 100000u) return IB200_ERR_INVALID_ARGUMENT;
     int rc = device_ok();
     if (rc != IB200_OK) return rc;
-    if ((rc = prepare_header(workspace, stream))) return rc;
     IB200_SET_BOUNDS(0, 0, 0, 0, 0, 1, 32, static_cast<int*>(workspace), stream);
     wait_expiry_probe_kernel<<<1, 128, 0, stream>>>(static_cast<int*>(workspace), 1000ull * limit_us);
     return launch_status();

@@ -2,8 +2,7 @@
 //   * split_bf16   fp32 x -> (hi, lo) bf16 pair with hi = bf16(x), lo = bf16(x - hi); the
 //                  fp32-I/O kernels multiply such pairs in three bf16 MMAs
 //   * bwd_prepass  one launch ahead of the backward main kernel: -delta[row] = -sum_d O[row,d] * dO[row,d] (and
-//                  -lse*log2e beside it), the zeroing of the dQ accumulator, the workspace header and (fp32 I/O) the
-//                  operand splits; delta is the reference's
+//                  -lse*log2e beside it), the zeroing of the dQ accumulator and (fp32 I/O) the operand splits; delta is the reference's
 //                  dot = sum_j dP_ij P_ij (src/inferno/gradfn/softmaxbackward.h:101-109)
 //                  rewritten so that it needs no [T,T] matrix
 //   * dq_finish    dQ = scale * accumulator, cast to the output type; the scale is
@@ -17,6 +16,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "sm100_ptx.cuh"
+
 namespace ib200 {
 
 // cudaError_t of the most recent failing CUDA call on this host thread (what ib200_last_cuda_error returns).
@@ -29,6 +30,21 @@ inline bool cuda_ok(cudaError_t e) {
 }
 constexpr int kErrCuda = 5;      // IB200_ERR_CUDA
 inline int launch_status() { return cuda_ok(cudaGetLastError()) ? 0 : kErrCuda; }
+// Launch that may overlap its predecessor's tail (the kernel calls pdl_wait before it touches global memory).
+template <auto KERNEL, class... Args>
+inline int launch_pdl(dim3 grid, dim3 block, size_t smem, cudaStream_t stream, const Args&... args) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cuda_ok(cudaLaunchKernelEx(&cfg, KERNEL, args...)) ? 0 : kErrCuda;
+}
 
 // Where the rows of a [B, H, T, D] operand live: element strides of the batch, head and token axes
 // (the D elements of a row are contiguous).  Dense row-major is {H*T*D, T*D, D}; a q/k/v slice of a packed
@@ -81,28 +97,20 @@ __device__ __forceinline__ void split_bf16_block(const SplitJob& job, int z, int
     }
 }
 
-// Workspace header (see attn_api.cu): word 0 = sticky device status, word 1 = draw counter of the persistent kernels
-// (zero at every launch), word 3 = "status word is valid" mark for a workspace that arrives uninitialised.
-constexpr int kHeaderMagic = 0x1b200a77;
-__device__ __forceinline__ void prepare_header(int* hdr) {
-    if (hdr[3] != kHeaderMagic) { hdr[0] = 0; hdr[3] = kHeaderMagic; }
-    hdr[1] = 0;
-}
-
-// Forward pre-pass of the fp32-I/O path: q, k, v -> hi / lo copies (grid z = operand), and the header.
-__global__ void __launch_bounds__(kAuxThreads) split_bf16_kernel(SplitJob job, int* header, int T, int D) {
-    if (header && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0) prepare_header(header);
+// Forward pre-pass of the fp32-I/O path: q, k, v -> hi / lo copies (grid z = operand).
+__global__ void __launch_bounds__(kAuxThreads) split_bf16_kernel(SplitJob job, int T, int D) {
+    pdl_wait();
+    pdl_trigger();
     split_bf16_block(job, blockIdx.z, T, D);
 }
 
 // n_ops operands (3 or 4) in one launch.
-inline int launch_split_bf16(const SplitJob& job, int n_ops, int* header, long heads, int T, int D, cudaStream_t stream) {
+inline int launch_split_bf16(const SplitJob& job, int n_ops, long heads, int T, int D, cudaStream_t stream) {
     const int n8 = T * (D / 8);
     int bx = (n8 + kAuxThreads - 1) / kAuxThreads;
     if (bx > 64) bx = 64;                                    // grid-stride inside a head beyond that
     dim3 grid(bx, static_cast<unsigned>(heads), static_cast<unsigned>(n_ops));
-    split_bf16_kernel<<<grid, kAuxThreads, 0, stream>>>(job, header, T, D);
-    return launch_status();
+    return launch_pdl<split_bf16_kernel>(grid, kAuxThreads, 0, stream, job, T, D);
 }
 
 // Dense casts between fp32 and bf16 (round to nearest even), 8 elements per thread: for callers whose tensors are
@@ -189,7 +197,7 @@ __device__ __forceinline__ void delta_block(const void* __restrict__ o_, const v
 }
 
 // The backward's one pre-pass launch.  Grid y = head; grid z selects the job:
-//   z = 0      -delta and -lse*log2e of the head's rows (delta_block), and the workspace header
+//   z = 0      -delta and -lse*log2e of the head's rows (delta_block)
 //   z = 1      zeroes the head's slice of the fp32 dQ accumulator (the main kernel adds into it)
 //   z = 2..5   (fp32 I/O only) q, k, v, dO -> hi / lo bf16 copies
 // grid x = blocks of 64 rows, which is what delta_block needs; the other jobs stride over it.
@@ -201,14 +209,14 @@ struct BwdPrepassJob {
     float* nlse2;
     RowLayout lo, ldo;
     float4* dq_acc;        // dense [heads, T, D] fp32
-    int* header;
     SplitJob split;        // used when F32
 };
 template <int D, bool F32>
 __global__ void __launch_bounds__(kAuxThreads) bwd_prepass_kernel(BwdPrepassJob job, int T, int T_pad) {
     const int z = blockIdx.z;
+    pdl_wait();
+    pdl_trigger();
     if (z == 0) {
-        if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) prepare_header(job.header);
         delta_block<D, F32>(job.o, job.dO, job.lse, job.ndelta, job.nlse2, job.lo, job.ldo, T, T_pad);
     } else if (z == 1) {
         const long n4 = static_cast<long>(T) * (D / 4);                      // float4 chunks of this head's accumulator slice
@@ -224,8 +232,7 @@ template <int D, bool F32>
 inline int launch_bwd_prepass(const BwdPrepassJob& job, long heads, int T, int T_pad, cudaStream_t stream) {
     constexpr int RPB = kAuxThreads / (D / (F32 ? 4 : 8));
     dim3 grid((T_pad + RPB * 4 - 1) / (RPB * 4), static_cast<unsigned>(heads), F32 ? 6 : 2);
-    bwd_prepass_kernel<D, F32><<<grid, kAuxThreads, 0, stream>>>(job, T, T_pad);
-    return launch_status();
+    return launch_pdl<bwd_prepass_kernel<D, F32>>(grid, kAuxThreads, 0, stream, job, T, T_pad);
 }
 
 // out[row, :] = scale * acc[row, :], 8 elements per thread; acc is dense [heads, T, D], out follows `lout`.
@@ -276,6 +283,7 @@ template <int D, bool F32>
 inline int launch_dq_finish(const float* acc, void* out, float scale, const RowLayout& lout, long heads, int T, cudaStream_t stream) {
     const int n8 = T * (D / 8);
     dim3 grid((n8 + kAuxThreads * 4 - 1) / (kAuxThreads * 4), static_cast<unsigned>(heads), 1);
+    // an ordinary launch: thousands of small blocks that wait for the main kernel's tail made the pair 3-10 % slower
     dq_finish_kernel<D, F32><<<grid, kAuxThreads, 0, stream>>>(reinterpret_cast<const float4*>(acc), out, scale, lout, T);
     return launch_status();
 }

@@ -12,8 +12,8 @@
 //   * a CTA's launch, barrier set-up, TMEM allocation and tear-down are paid once per SM instead of once per item.
 // A CTA launched per item spends about 11 us outside its steady state (17 % of an average item at T = 4096; measured
 // on the one-CTA-per-item form this kernel replaced).
-// Items are drawn, not assigned: a CTA starts on item blockIdx.x and its TMA thread draws every further index from a
-// counter in global memory (ItemRing in sm100_ptx.cuh hands it to the other roles).  The list runs over groups of
+// Items are drawn, not assigned: a CTA starts on item blockIdx.x and its TMA thread takes over the items of CTAs that have not
+// been launched yet (ItemRing in sm100_ptx.cuh hands them to the other roles).  The list runs over groups of
 // consecutive heads (locate_item) so that the CTAs share the Q / dO tiles and the fp32 dQ accumulator of few heads in L2 at
 // a time, and inside a group from key tile 0 (the longest walk) to the last.
 #pragma once
@@ -29,7 +29,7 @@ attn_bwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                         const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_v_lo,
                         const __grid_constant__ CUtensorMap tm_do, const __grid_constant__ CUtensorMap tm_do_lo,
                         const __grid_constant__ CUtensorMap tm_dk, const __grid_constant__ CUtensorMap tm_dv,
-                        const __grid_constant__ CUtensorMap tm_dq, BwdParams prm, int n_items, int n_groups, int* next_item) {
+                        const __grid_constant__ CUtensorMap tm_dq, BwdParams prm, int n_items, int n_groups) {
     constexpr int D = TR::D, BKV = TR::BKV, BQ = TR::BQ, NS = TR::NS, NB = TR::NB;
     constexpr bool SPLIT = TR::SPLIT;
     // groups of four queries (of the eight a compute thread handles per block) whose lse / delta values are fetched early;
@@ -64,9 +64,11 @@ attn_bwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     uint64_t* dkv_free = dkv_full + 1;      // [1]   drain warps (4): dK, dV read out of TMEM
     uint64_t* dp_full = dkv_free + 1;       // [NB]  MMA commit: dP^T of a block is in TMEM
     uint64_t* item_bars = dp_full + NB;     // [4]   item ring: full[2], empty[2]
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(item_bars + 4);
+    uint64_t* clc_bar = item_bars + 4;      // [1]   answer to the request for another item
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(item_bars + 5);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     const ItemRing items{item_bars, item_bars + 2, abort_flag + 1};
+    const ItemSource source{reinterpret_cast<uint4*>(smem + TR::OFF_BAR + 496), clc_bar};
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int T = prm.T;
@@ -97,6 +99,7 @@ attn_bwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
         }
         mbar_init(dkv_full, 1);
         mbar_init(dkv_free, 4);
+        mbar_init(clc_bar, 1);
         item_ring_init(items, 13);               // readers: the MMA warp, eight compute warps, four drain warps
         fence_mbar_init();
     }
@@ -110,6 +113,7 @@ attn_bwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
+    pdl_wait();
 
     if (warp >= 12) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
@@ -125,8 +129,7 @@ attn_bwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
             for (int idx = blockIdx.x; idx < n_items; ++ni) {
                 if (*abort_flag != 0) break;
                 const Item item = decode(idx);
-                // draw the next item now; the value is needed (and published to the other roles) only after this item's K / V loads
-                const int drawn = atomicAdd(next_item, 1);
+                item_request(source);
                 if (ni > 0) mbar_wait(dkv_full, (ni - 1) & 1, ab, 12);          // the previous item's MMAs have finished with K, V
                 mbar_arrive_expect_tx(kv_full, 2 * TR::KV_TILE);
                 // panel p of a tile: columns 64p.. of a bf16 operand, or (fp32 I/O) the hi / lo half of the bf16 pair
@@ -135,7 +138,7 @@ attn_bwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                     tma_load_4d(sK + p * TR::KV_PANEL, (SPLIT && p) ? &tm_k_lo : &tm_k, kv_full, col(p), item.n * BKV, item.hd, item.bt);
                     tma_load_4d(sV + p * TR::KV_PANEL, (SPLIT && p) ? &tm_v_lo : &tm_v, kv_full, col(p), item.n * BKV, item.hd, item.bt);
                 }
-                idx = static_cast<int>(gridDim.x) + drawn;
+                idx = item_take(source, ni, n_items, ab);
                 item_ring_publish(items, ni, idx, ab);
                 for (int it = 0; it < item.nblk; ++it, ++g) {
                     const int s = g % NS;
@@ -152,6 +155,8 @@ attn_bwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                     bulk_load_1d(sVec + s * 2 * BQ + BQ, prm.ndelta + voff, BQ * 4, &qdo_full[s]);
                 }
             }
+            pdl_trigger();      // this CTA's last loads are out: the next kernel may start as the SMs empty (triggered at the start instead, the next
+                                // kernel's waiting CTAs cost the backward 5-10 %)
         }
     } else if (warp == 13) {
         // ------------------------------ MMA issuer (converged warp, one elected lane issues) ------------------------------

@@ -12,9 +12,9 @@
 // the one-CTA-per-item form this kernel replaced): 20 % of an average item at T = 4096 and half of one at T = 1024;
 // here most of it runs under another item's work.
 // All mbarrier phases run on from item to item; each role derives them from its own counters.
-// Items are drawn, not assigned: a CTA starts on item blockIdx.x and its TMA thread draws every further index from a
-// counter in global memory (ItemRing in sm100_ptx.cuh hands it to the other roles), so CTAs that drew short walks draw more
-// of them.  The list runs over groups of consecutive heads (locate_item) so that the CTAs share the K / V tiles of few
+// Items are drawn, not assigned: a CTA starts on item blockIdx.x and its TMA thread takes over the items of CTAs that have not
+// been launched yet (ItemRing in sm100_ptx.cuh hands them to the other roles), so CTAs that drew short walks draw more
+// of them.  That makes a bf16 forward one launch: a counter in memory needed a launch ahead of it to be zeroed.  The list runs over groups of consecutive heads (locate_item) so that the CTAs share the K / V tiles of few
 // heads in L2 at a time, and inside a group from the longest walk to the shortest.
 #pragma once
 
@@ -36,7 +36,6 @@ struct FwdPersistParams {
     int n_items;        // pairs_per_head * BH
     int pairs_per_head; // ceil(T / 256)
     int n_groups;       // head groups of the item list (see locate_item)
-    int* next_item;     // draw counter in global memory, zero at launch
 };
 
 template <class TR>
@@ -65,9 +64,11 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     uint64_t* o_free = o_full + 2;          // [2]   the epilogue has read O_i out of TMEM (4 warps)
     uint64_t* stage_free = o_free + 2;      // [1]   the TMA store has read the staging tile
     uint64_t* ring_bars = stage_free + 1;   // [4]   item ring: full[2], empty[2]
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ring_bars + 4);
+    uint64_t* clc_bar = ring_bars + 4;      // [1]   answer to the request for another item
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ring_bars + 5);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     const ItemRing ring{ring_bars, ring_bars + 2, abort_flag + 1};
+    const ItemSource source{reinterpret_cast<uint4*>(smem + TR::OFF_BAR + 496), clc_bar};
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int T = prm.T;
@@ -104,6 +105,7 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
             mbar_init(&o_full[i], 1); mbar_init(&o_free[i], 4);
         }
         mbar_init(stage_free, 1);
+        mbar_init(clc_bar, 1);
         item_ring_init(ring, 9);                 // readers: the MMA warp and the eight softmax warps
         fence_mbar_init();
     }
@@ -116,6 +118,7 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
+    pdl_wait();
 
     if (warp >= 8) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
@@ -128,8 +131,7 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
             for (int idx = blockIdx.x; idx < pp.n_items; ++n) {
                 if (*abort_flag != 0) break;
                 const Item it = decode(idx);
-                // draw the next item now; the value is needed (and published to the other roles) only after this item's first loads
-                const int drawn = atomicAdd(pp.next_item, 1);
+                item_request(source);
                 if (n > 0) mbar_wait(q_free, (n - 1) & 1, ab, 12);
                 const int q_tiles = (it.nkv1 > 0) ? 2 : 1;
                 mbar_arrive_expect_tx(q_full, (q_tiles + 1) * TR::TILE_BYTES);
@@ -141,7 +143,7 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                         tma_load_4d(sQ + TR::TILE_BYTES + p * TR::PANEL_BYTES, (TR::SPLIT && p) ? &tm_q_lo : &tm_q, q_full, col(p), it.m1 * BM, it.hd, it.bt);
                 for (int p = 0; p < TR::NP; ++p)
                     tma_load_4d(sK + (G % KS) * TR::TILE_BYTES + p * TR::PANEL_BYTES, (TR::SPLIT && p) ? &tm_k_lo : &tm_k, q_full, col(p), 0, it.hd, it.bt);
-                idx = static_cast<int>(gridDim.x) + drawn;
+                idx = item_take(source, n, pp.n_items, ab);
                 item_ring_publish(ring, n, idx, ab);
                 for (int j = 0; j < it.n_iter; ++j, ++G) {
                     const int s = G % KS;
@@ -157,6 +159,8 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                         tma_load_4d(sV + s * TR::TILE_BYTES + p * TR::PANEL_BYTES, (TR::SPLIT && p) ? &tm_v_lo : &tm_v, &kv_full[s], col(p), j * BN, it.hd, it.bt);
                 }
             }
+            pdl_trigger();      // this CTA's last loads are out: the next kernel may start as the SMs empty (triggered at the start instead, the next
+                                // kernel's waiting CTAs cost the backward 5-10 %)
         }
     } else if (warp == 8) {
         // ------------------------------ MMA issuer (converged warp, one elected lane issues) ------------------------------

@@ -43,8 +43,9 @@ struct Abi {
     decltype(&ib200_attn_workspace_bytes) workspace_bytes = nullptr;
     decltype(&ib200_attn_fwd_strided) attn_fwd = nullptr;
     decltype(&ib200_attn_bwd_strided) attn_bwd = nullptr;
-    decltype(&ib200_linear_fwd) linear_fwd = nullptr;
-    decltype(&ib200_linear_bwd) linear_bwd = nullptr;
+    decltype(&ib200_linear_workspace_bytes) linear_workspace_bytes = nullptr;
+    decltype(&ib200_linear_fwd_ws) linear_fwd = nullptr;
+    decltype(&ib200_linear_bwd_ws) linear_bwd = nullptr;
     decltype(&ib200_attn_set_timing_events) set_timing_events = nullptr;
     decltype(&ib200_status_string) status_string = nullptr;
     PyObject* error_class = nullptr;      // the package's exception type, constructed from (status, where)
@@ -381,6 +382,9 @@ void check_bf16_cuda(const Tensor& t, const char* name) {
     TORCH_CHECK_TYPE(t.scalar_type() == at::kBFloat16, "linear: ", name, " must be bfloat16");
 }
 
+// The stream's workspace begins with the attention calls' header (their sticky status); the projections use what follows it.
+constexpr size_t kHeaderBytes = 256;
+
 Tensor linear_forward(const Tensor& x, const Tensor& w, const Tensor& bias) {
     check_bf16_cuda(x, "x");
     check_bf16_cuda(w, "w");
@@ -388,21 +392,33 @@ Tensor linear_forward(const Tensor& x, const Tensor& w, const Tensor& bias) {
     const c10::cuda::CUDAGuard guard(x.device());
     const int64_t K = w.size(0), N = w.size(1);
     const Tensor x2 = x.reshape({-1, K}).contiguous(), wc = w.contiguous();
-    const Tensor b = bias.defined() ? bias.to(at::kFloat).contiguous() : Tensor();
+    Tensor b = bias;
+    if (b.defined() && b.scalar_type() != at::kBFloat16) b = b.to(at::kFloat);
+    if (b.defined()) b = b.contiguous();
     auto shape = x.sizes().vec();
     shape.back() = N;
     Tensor y = at::empty(shape, x.options());
-    check_status(g_abi.linear_fwd(x2.data_ptr(), wc.data_ptr(), b.defined() ? b.data_ptr<float>() : nullptr, y.data_ptr(), static_cast<int>(x2.size(0)),
-                                  static_cast<int>(K), static_cast<int>(N),
-                                  reinterpret_cast<ib200_stream_t>(c10::cuda::getCurrentCUDAStream(x.device().index()).stream())),
-                 "ib200_linear_fwd");
+    const int M = static_cast<int>(x2.size(0));
+    const size_t bytes = g_abi.linear_workspace_bytes(M, static_cast<int>(K), static_cast<int>(N), IB200_PASS_FWD);
+    cudaStream_t stream = c10::cuda::getCurrentCUDAStream(x.device().index()).stream();
+    std::unique_lock<std::mutex> lock;
+    void* scratch = nullptr;
+    if (bytes) {
+        Workspace& ws = workspace_of(x.device().index(), stream);
+        lock = std::unique_lock<std::mutex>(ws.launching);
+        reserve(ws, kHeaderBytes + bytes, x.device());
+        scratch = static_cast<char*>(ws.buf.data_ptr()) + kHeaderBytes;
+    }
+    check_status(g_abi.linear_fwd(x2.data_ptr(), wc.data_ptr(), b.defined() ? b.data_ptr() : nullptr, b.defined() ? dtype_code(b) : IB200_DTYPE_F32,
+                                  y.data_ptr(), M, static_cast<int>(K), static_cast<int>(N), scratch, bytes, reinterpret_cast<ib200_stream_t>(stream)),
+                 "ib200_linear_fwd_ws");
     return y;
 }
 
 struct LinearGrads {
     Tensor dx, dw, db;
 };
-LinearGrads linear_backward(const Tensor& x, const Tensor& w, const Tensor& dy, bool need_dx, bool need_dw, bool need_db) {
+LinearGrads linear_backward(const Tensor& x, const Tensor& w, const Tensor& dy, bool need_dx, bool need_dw, bool need_db, bool db_bf16) {
     check_bf16_cuda(x, "x");
     check_bf16_cuda(w, "w");
     check_bf16_cuda(dy, "dy");
@@ -410,15 +426,21 @@ LinearGrads linear_backward(const Tensor& x, const Tensor& w, const Tensor& dy, 
     const c10::cuda::CUDAGuard guard(x.device());
     const int64_t K = w.size(0), N = w.size(1);
     const Tensor x2 = x.reshape({-1, K}).contiguous(), dy2 = dy.reshape({-1, N}).contiguous(), wc = w.contiguous();
+    const int M = static_cast<int>(x2.size(0));
     LinearGrads g;
     if (need_dx) g.dx = at::empty(x.sizes(), x.options());
     if (need_dw) g.dw = at::empty({K, N}, x.options());
-    if (need_db) g.db = at::empty({N}, x.options().dtype(at::kFloat));
+    if (need_db) g.db = at::empty({N}, x.options().dtype(db_bf16 ? at::kBFloat16 : at::kFloat));
+    const size_t bytes = g_abi.linear_workspace_bytes(M, static_cast<int>(K), static_cast<int>(N), IB200_PASS_BWD);
+    cudaStream_t stream = c10::cuda::getCurrentCUDAStream(x.device().index()).stream();
+    Workspace& ws = workspace_of(x.device().index(), stream);
+    std::lock_guard<std::mutex> lock(ws.launching);
+    reserve(ws, kHeaderBytes + bytes, x.device());
     auto ptr = [](const Tensor& t) -> void* { return t.defined() ? t.data_ptr() : nullptr; };
-    check_status(g_abi.linear_bwd(x2.data_ptr(), wc.data_ptr(), dy2.data_ptr(), ptr(g.dx), ptr(g.dw), static_cast<float*>(ptr(g.db)),
-                                  static_cast<int>(x2.size(0)), static_cast<int>(K), static_cast<int>(N),
-                                  reinterpret_cast<ib200_stream_t>(c10::cuda::getCurrentCUDAStream(x.device().index()).stream())),
-                 "ib200_linear_bwd");
+    check_status(g_abi.linear_bwd(x2.data_ptr(), wc.data_ptr(), dy2.data_ptr(), ptr(g.dx), ptr(g.dw), ptr(g.db), db_bf16 ? IB200_DTYPE_BF16 : IB200_DTYPE_F32, M,
+                                  static_cast<int>(K), static_cast<int>(N), static_cast<char*>(ws.buf.data_ptr()) + kHeaderBytes, bytes,
+                                  reinterpret_cast<ib200_stream_t>(stream)),
+                 "ib200_linear_bwd_ws");
     return g;
 }
 
@@ -433,10 +455,10 @@ struct LinearBackward : torch::autograd::Node {
         const Tensor tx = x.unpack(), tw = w.unpack();
         at::AutoDispatchBelowADInplaceOrView below;
         LinearGrads g = linear_backward(tx, tw, grads[0], task_should_compute_output(0), task_should_compute_output(1),
-                                        has_bias && task_should_compute_output(2));
+                                        has_bias && task_should_compute_output(2), bias_type == at::kBFloat16);
         out[0] = g.dx;
         out[1] = g.dw;
-        if (g.db.defined()) out[2] = g.db.to(bias_type);
+        if (g.db.defined()) out[2] = g.db.to(bias_type);      // fp32 and bf16 come in the right type
         return out;
     }
     void release_variables() override { x.reset_data(); w.reset_data(); }
@@ -530,8 +552,9 @@ PyObject* py_bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
         get(g_abi.workspace_bytes, "ib200_attn_workspace_bytes");
         get(g_abi.attn_fwd, "ib200_attn_fwd_strided");
         get(g_abi.attn_bwd, "ib200_attn_bwd_strided");
-        get(g_abi.linear_fwd, "ib200_linear_fwd");
-        get(g_abi.linear_bwd, "ib200_linear_bwd");
+        get(g_abi.linear_workspace_bytes, "ib200_linear_workspace_bytes");
+        get(g_abi.linear_fwd, "ib200_linear_fwd_ws");
+        get(g_abi.linear_bwd, "ib200_linear_bwd_ws");
         get(g_abi.set_timing_events, "ib200_attn_set_timing_events");
         get(g_abi.status_string, "ib200_status_string");
         Py_INCREF(a[1]);
@@ -652,7 +675,7 @@ PyObject* py_linear_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
         {
             pybind11::gil_scoped_release nogil;
             at::AutoDispatchBelowADInplaceOrView below;
-            g = linear_backward(x, w, dy, need_dx, need_dw, need_db);
+            g = linear_backward(x, w, dy, need_dx, need_dw, need_db, false);
         }
         return wrap_tuple({&g.dx, &g.dw, &g.db});
     });

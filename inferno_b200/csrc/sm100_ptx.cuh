@@ -36,6 +36,16 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// Header of a workspace: word 0 = device status (sticky until the host has read it), word 3 = a mark that says word 0 is a status.
+// A workspace arrives uninitialised and no launch prepares it: whoever has something to report sets the mark, and a first
+// report replaces whatever word 0 held.
+constexpr int kHeaderMagic = 0x1b200a77;
+__device__ __forceinline__ void report_status(int* header, int code) {
+    if (!header) return;
+    if (atomicExch(header + 3, kHeaderMagic) != kHeaderMagic) atomicExch(header, code);
+    else atomicCAS(header, 0, code);
+}
+
 enum : int {
     kDevOk = 0,
     kDevTimeoutBase = 100,   // 100 + site id of the wait that gave up
@@ -62,12 +72,13 @@ __constant__ BoundsInfo c_bounds;
 enum : int { kBndTmaLoad = 1, kBndTmaStore = 2, kBndTmaReduce = 3, kBndBulkLoad = 4, kBndTmemLd = 5, kBndTmemSt = 6, kBndMmaDesc = 7, kBndSwizzle = 8 };
 __device__ __forceinline__ bool bounds_ok(bool cond, int kind) {
     if (cond) return true;
-    if (c_bounds.status) atomicCAS(c_bounds.status, 0, kDevBoundsBase + kind);
+    report_status(c_bounds.status, kDevBoundsBase + kind);
     return false;
 }
 __device__ __forceinline__ bool smem_addr_ok(uint32_t saddr, uint32_t align) {
     uint32_t total;
     asm volatile("mov.u32 %0, %%total_smem_size;" : "=r"(total));
+    saddr &= 0xffffffu;                  // in a cluster the bits above are the CTA's rank
     return saddr < total && (saddr & (align - 1)) == 0;
 }
 __device__ __forceinline__ bool coords4_ok(int c0, int c1, int c2, int c3) {
@@ -126,24 +137,38 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
+// A wait for arrivals made by threads of the cluster's other CTA: the probes acquire at cluster scope.  (The CTA-scope wait
+// followed by fence.acq_rel.cluster held up the MMA issuer of a CTA pair for 1800 cycles per tile.)
+__device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
 // Returns false if the wait was abandoned (abort already raised, or limit hit).
 // The CTA abort flag lives in shared memory; it is polled only every 64th failed try so that
 // spinning warps do not load the shared-memory pipe the MMAs and compute warps depend on.
 // `limit_ns` is a compile-time constant at every call site of the product kernels (mbar_wait below);
 // only the wait-expiry self-test kernel passes a run-time value.
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait_limit(uint64_t* bar, uint32_t parity, const AbortCtx& ab, int site, unsigned long long limit_ns) {
-    if (mbar_test_wait(bar, parity)) return true;
+    if (!CLUSTER && mbar_test_wait(bar, parity)) return true;
     uint32_t spins = 0;
     unsigned long long t_start = 0;
     while (true) {
-        if (mbar_try_wait(bar, parity)) return true;
+        if (CLUSTER ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity)) return true;
         if ((++spins & 63u) == 0) {
             if (*ab.cta_flag != 0) return false;
             const unsigned long long now = global_timer_ns();
             if (t_start == 0) t_start = now;
             if (spins > kSpinLimit || now - t_start > limit_ns) {
                 *ab.cta_flag = 1;
-                if (ab.status) atomicCAS(ab.status, 0, kDevTimeoutBase + site);
+                report_status(ab.status, kDevTimeoutBase + site);
                 return false;
             }
         }
@@ -152,13 +177,49 @@ __device__ __forceinline__ bool mbar_wait_limit(uint64_t* bar, uint32_t parity, 
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const AbortCtx& ab, int site) {
     return mbar_wait_limit(bar, parity, ab, site, kWaitLimitNs);
 }
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, const AbortCtx& ab, int site) {
+    return mbar_wait_limit<true>(bar, parity, ab, site, kWaitLimitNs);
+}
+
+// Generic-proxy accesses to shared memory -> ordered before later ones of the async proxy (TMA, MMA).
+__device__ __forceinline__ void fence_proxy_async_smem() {
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+
+// ---- launch overlap (programmatic dependent launch) -------------------------------
+// A kernel launched with the programmatic-serialization attribute may start while its predecessor in the stream still runs;
+// pdl_wait returns once that predecessor has completed and its writes are visible, and every access to global memory (reads,
+// writes, TMA) comes after it.  pdl_trigger lets the successor start: its CTAs take the SMs this grid leaves and set up
+// (barriers, tensor memory, descriptor fetches) under this grid's tail.  Both are no-ops for an ordinary launch.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---- work items of a persistent CTA ---------------------------------------------
-// Every CTA starts on item blockIdx.x and then draws items from a counter in global memory (zero at launch), so a CTA
-// that drew light items simply draws more of them.  One thread of the CTA (the TMA producer, which runs furthest ahead)
-// draws; the other roles read what it drew through a two-slot ring in shared memory: slot n & 1 holds the item that
-// follows the CTA's n-th item, full[] (count 1) says it has been written, empty[] (count = reading warps) that every
-// role has read it.  An index >= the item count ends every role's loop.
+// The grid has one CTA per item; only as many as fit become resident.  A resident CTA starts on item blockIdx.x and then
+// takes over the items of CTAs that have not been launched yet, by cancelling their launch (clusterlaunchcontrol), so a CTA
+// that got light items simply takes more of them, in the order of the list, and no counter in memory is needed.  One thread
+// of the CTA (the TMA producer, which runs furthest ahead) asks; the other roles read what it got through a two-slot ring in
+// shared memory: slot n & 1 holds the item that follows the CTA's n-th item, full[] (count 1) says it has been written,
+// empty[] (count = reading warps) that every role has read it.  An index >= the item count ends every role's loop.
+__device__ __forceinline__ void clc_try_cancel(uint4* response, uint64_t* bar) {
+    asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(smem_u32(response)), "r"(smem_u32(bar))
+                 : "memory");
+}
+// blockIdx.x of the cancelled CTA, or `none` when there was nothing left to cancel (then no further request may be made)
+__device__ __forceinline__ int clc_cancelled_ctaid(const uint4* response, int none) {
+    uint32_t ok, x;
+    asm volatile(
+        "{\n\t.reg .b128 r;\n\t.reg .pred p;\n\t"
+        "ld.shared.b128 r, [%2];\n\t"
+        "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t"
+        "mov.u32 %1, 0;\n\t"
+        "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, r;\n\t}"
+        : "=r"(ok), "=r"(x)
+        : "r"(smem_u32(response))
+        : "memory");
+    return ok ? static_cast<int>(x) : none;
+}
 struct ItemRing {
     uint64_t* full;        // [2]
     uint64_t* empty;       // [2]
@@ -166,6 +227,20 @@ struct ItemRing {
 };
 __device__ __forceinline__ void item_ring_init(const ItemRing& r, uint32_t readers) {
     for (int s = 0; s < 2; ++s) { mbar_init(&r.full[s], 1); mbar_init(&r.empty[s], readers); }
+}
+// Producer thread: ask for the next item (the answer is needed only after the current item's first loads), and take it.
+struct ItemSource {
+    uint4* response;       // 16-byte aligned shared memory
+    uint64_t* bar;         // count 1
+};
+__device__ __forceinline__ void item_request(const ItemSource& src) {
+    fence_proxy_async_smem();                     // the previous answer has been read
+    mbar_arrive_expect_tx(src.bar, 16);
+    clc_try_cancel(src.response, src.bar);
+}
+__device__ __forceinline__ int item_take(const ItemSource& src, int n, int none, const AbortCtx& ab) {
+    if (!mbar_wait(src.bar, n & 1, ab, 16)) return none;
+    return clc_cancelled_ctaid(src.response, none);
 }
 // producer thread: the item after this CTA's n-th item is `next`
 __device__ __forceinline__ void item_ring_publish(const ItemRing& r, int n, int next, const AbortCtx& ab) {
@@ -207,11 +282,7 @@ __host__ __device__ __forceinline__ void locate_item(const HeadGroups& hg, int i
     bh = h0 + (r - unit_rank * hn);
 }
 
-// ---- proxy / tcgen05 fences ---------------------------------------------------
-// Generic-proxy writes to shared memory -> visible to the async proxy (TMA, MMA).
-__device__ __forceinline__ void fence_proxy_async_smem() {
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
+// ---- tcgen05 fences ---------------------------------------------------
 __device__ __forceinline__ void tc_fence_before_sync() {
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
 }
@@ -268,7 +339,7 @@ __device__ __forceinline__ void tma_store_3d(const CUtensorMap* m, const void* s
 }
 // 3-D tile reduction shared -> global: global[tile] += shared[tile], element type from the tensor map.
 __device__ __forceinline__ void tma_reduce_add_3d(const CUtensorMap* m, const void* smem_src, int c0, int c1, int c2) {
-    IB200_CHECKED(c0 == 0 && c1 >= 0 && c2 >= 0 && (c_bounds.relaxed || (c1 < c_bounds.dim[1] && c2 < c_bounds.rows3)) &&
+    IB200_CHECKED((c0 == 0 || (c_bounds.relaxed && c0 > 0 && (c0 & 7) == 0)) && c1 >= 0 && c2 >= 0 && (c_bounds.relaxed || (c1 < c_bounds.dim[1] && c2 < c_bounds.rows3)) &&
                   smem_addr_ok(smem_u32(smem_src), 128), kBndTmaReduce);
     asm volatile(
         "cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4}], [%1];"
@@ -326,6 +397,62 @@ __device__ __forceinline__ bool elect_one_lane() {
     uint32_t pred;
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(pred));
     return pred != 0;
+}
+
+// ---- CTA pairs (clusters of two) -----------------------------------------------------
+// With .cta_group::2 one MMA runs on the two SMs of a pair: each CTA holds its half of A's rows, its half of B's rows and its
+// half of the accumulator, at the same shared-memory and tensor-memory addresses; one thread of the even CTA issues.
+__device__ __forceinline__ uint32_t cluster_ctarank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+// Every thread of the cluster: arrive (release), then wait (acquire).
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Shared-memory address of the same variable in CTA `rank` of the cluster (shared::cluster window).
+__device__ __forceinline__ uint32_t mapa_u32(uint32_t saddr, uint32_t rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
+    return r;
+}
+// Arrival on a barrier of either CTA that hands over tensor memory only (whose reads tcgen05.wait::ld has completed and
+// tcgen05.fence orders): relaxed, because a release at cluster scope also waits for everything else the thread has written --
+// 3000 cycles when stores are on their way.
+__device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t cluster_addr) {
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+// Tile load into this CTA's shared memory whose bytes are counted on an mbarrier of either CTA of the pair.
+__device__ __forceinline__ void tma_load_3d_pair(void* smem_dst, const CUtensorMap* m, uint32_t bar_cluster_addr, int c0, int c1, int c2) {
+    IB200_CHECKED(coords4_ok(c0, c1, c2, 0) && smem_addr_ok(smem_u32(smem_dst), 1024), kBndTmaLoad);
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4, %5}], [%2];"
+        ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar_cluster_addr), "r"(c0), "r"(c1), "r"(c2)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_result, uint32_t ncols) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_result)), "r"(ncols) : "memory");
+}
+__device__ __forceinline__ void tmem_relinquish_pair() {
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+__device__ __forceinline__ void umma_ss_f16_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    IB200_CHECKED(smem_addr_ok(static_cast<uint32_t>(adesc & 0x3fffu) << 4, 16) && smem_addr_ok(static_cast<uint32_t>(bdesc & 0x3fffu) << 4, 16) &&
+                  tmem_addr_ok(d_tmem, ((idesc >> 17) & 0x3fu) << 3), kBndMmaDesc);
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// The pair's MMAs so far arrive, when complete, on the mbarrier at this offset in both CTAs.
+__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
+                 "h"(static_cast<uint16_t>(3)) : "memory");
 }
 
 // ---- descriptors ---------------------------------------------------------------
@@ -438,6 +565,12 @@ __device__ __forceinline__ float fmax3(float a, float b, float c) {
     float d;
     asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
     return d;
+}
+// 32 contiguous bytes (one sector) to global memory
+__device__ __forceinline__ void st_global_32b(void* p, const uint32_t (&v)[8]) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]),
+                 "r"(v[7])
+                 : "memory");
 }
 __device__ __forceinline__ uint64_t pack_f32x2(float lo, float hi) {
     uint64_t r;

@@ -62,3 +62,33 @@ def test_linear_module_autograd():
     assert rel(y.detach(), ref) < 1e-2
     assert rel(lin.bias.grad, torch.full((384,), 4 * 96.0, device="cuda")) < 1e-2
     assert x.grad is not None and lin.weight.grad is not None
+
+
+@pytest.mark.parametrize("M,K,N", [(8, 8, 8),              # less than one k-step, one corner of a tile
+                                   (256, 64, 256),         # exactly one tile of a CTA pair
+                                   (264, 72, 520),         # one step past it in every direction
+                                   (136, 4104, 264),       # forward cut along K, ragged last slice
+                                   (4104, 136, 264),       # weight gradient cut along K, ragged last slice
+                                   (1000, 768, 768), (20000, 256, 512),
+                                   (9480, 1032, 2056)])    # more tiles than CTA pairs in dX, dW's slices even out the load
+def test_tile_edges_and_split_products(M, K, N):
+    """Every output has one bf16 rounding on top of fp32 sums: at most 2^-9 of each value, so 2^-9 of the norm; the
+    summation error (2^-24 sqrt(K) at K <= 20000) is far below the factor of 1.5 left for it."""
+    g = torch.Generator(device="cuda").manual_seed(3 * M + K + N)
+    x = torch.randn(M, K, device="cuda", generator=g).to(torch.bfloat16).requires_grad_()
+    lin = L.Linear(K, N).cuda().to(torch.bfloat16)
+    with torch.no_grad():
+        lin.bias.copy_(torch.randn(N, device="cuda", generator=g))
+    dy = torch.randn(M, N, device="cuda", generator=g).to(torch.bfloat16)
+    y = lin(x)
+    dx, dw, db = torch.autograd.grad(y, (x, lin.weight, lin.bias), dy)
+    _, _, db32 = L.linear_backward(x.detach(), lin.weight.detach(), dy, need_dx=False)
+    _, dw1, _ = L.linear_backward(x.detach(), lin.weight.detach(), dy, need_dx=False, need_db=False)
+    torch.cuda.synchronize()
+    xd, wd, dyd = x.detach().double(), lin.weight.detach().double(), dy.double()
+    tol = 1.5 * 2.0 ** -9
+    assert rel(y.double(), xd @ wd + lin.bias.detach().double()) < tol
+    assert rel(dx.double(), dyd @ wd.t()) < tol
+    assert rel(dw.double(), xd.t() @ dyd) < tol and rel(dw1.double(), xd.t() @ dyd) < tol
+    assert db.dtype == torch.bfloat16 and rel(db.double(), dyd.sum(0)) < tol
+    assert rel(db32.double(), dyd.sum(0)) < 1e-5
