@@ -129,7 +129,6 @@ attn_bwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
             for (int idx = blockIdx.x; idx < n_items; ++ni) {
                 if (*abort_flag != 0) break;
                 const Item item = decode(idx);
-                item_request(source);
                 if (ni > 0) mbar_wait(dkv_full, (ni - 1) & 1, ab, 12);          // the previous item's MMAs have finished with K, V
                 mbar_arrive_expect_tx(kv_full, 2 * TR::KV_TILE);
                 // panel p of a tile: columns 64p.. of a bf16 operand, or (fp32 I/O) the hi / lo half of the bf16 pair
@@ -138,12 +137,11 @@ attn_bwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                     tma_load_4d(sK + p * TR::KV_PANEL, (SPLIT && p) ? &tm_k_lo : &tm_k, kv_full, col(p), item.n * BKV, item.hd, item.bt);
                     tma_load_4d(sV + p * TR::KV_PANEL, (SPLIT && p) ? &tm_v_lo : &tm_v, kv_full, col(p), item.n * BKV, item.hd, item.bt);
                 }
-                idx = item_take(source, ni, n_items, ab);
-                item_ring_publish(items, ni, idx, ab);
                 for (int it = 0; it < item.nblk; ++it, ++g) {
                     const int s = g % NS;
                     const int m = item.m0 + it;
                     mbar_wait(&qdo_empty[s], ((g / NS) & 1) ^ 1, ab, 10);
+                    if (it == item.nblk - 1) item_request(source);      // NS blocks before the item's end (see ItemSource)
                     mbar_arrive_expect_tx(&qdo_full[s], 2 * TR::Q_TILE + 2 * BQ * 4);
                     for (int p = 0; p < TR::NP; ++p) {
                         tma_load_4d(sQ + s * TR::Q_TILE + p * TR::Q_PANEL, (SPLIT && p) ? &tm_q_lo : &tm_q, &qdo_full[s], col(p), m * BQ, item.hd, item.bt);
@@ -154,6 +152,8 @@ attn_bwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                     bulk_load_1d(sVec + s * 2 * BQ, prm.nlse2 + voff, BQ * 4, &qdo_full[s]);
                     bulk_load_1d(sVec + s * 2 * BQ + BQ, prm.ndelta + voff, BQ * 4, &qdo_full[s]);
                 }
+                idx = item_take(source, ni, n_items, ab);
+                item_ring_publish(items, ni, idx, ab);
             }
             pdl_trigger();      // this CTA's last loads are out: the next kernel may start as the SMs empty (triggered at the start instead, the next
                                 // kernel's waiting CTAs cost the backward 5-10 %)

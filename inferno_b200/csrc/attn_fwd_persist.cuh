@@ -131,7 +131,6 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
             for (int idx = blockIdx.x; idx < pp.n_items; ++n) {
                 if (*abort_flag != 0) break;
                 const Item it = decode(idx);
-                item_request(source);
                 if (n > 0) mbar_wait(q_free, (n - 1) & 1, ab, 12);
                 const int q_tiles = (it.nkv1 > 0) ? 2 : 1;
                 mbar_arrive_expect_tx(q_full, (q_tiles + 1) * TR::TILE_BYTES);
@@ -143,12 +142,11 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                         tma_load_4d(sQ + TR::TILE_BYTES + p * TR::PANEL_BYTES, (TR::SPLIT && p) ? &tm_q_lo : &tm_q, q_full, col(p), it.m1 * BM, it.hd, it.bt);
                 for (int p = 0; p < TR::NP; ++p)
                     tma_load_4d(sK + (G % KS) * TR::TILE_BYTES + p * TR::PANEL_BYTES, (TR::SPLIT && p) ? &tm_k_lo : &tm_k, q_full, col(p), 0, it.hd, it.bt);
-                idx = item_take(source, n, pp.n_items, ab);
-                item_ring_publish(ring, n, idx, ab);
                 for (int j = 0; j < it.n_iter; ++j, ++G) {
                     const int s = G % KS;
                     const bool has_k = (j + 1) < it.n_iter;
                     mbar_wait(&kv_empty[s], ((G / KS) & 1) ^ 1, ab, 10);
+                    if (!has_k) item_request(source);        // KS key tiles before the item's end (see ItemSource)
                     if (j == KS - 1) mbar_wait(k0_free, n & 1, ab, 11);         // K_KS reuses the slot of K_0
                     mbar_arrive_expect_tx(&kv_full[s], (has_k ? 2 : 1) * TR::TILE_BYTES);
                     if (has_k)
@@ -158,6 +156,8 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                     for (int p = 0; p < TR::NP; ++p)
                         tma_load_4d(sV + s * TR::TILE_BYTES + p * TR::PANEL_BYTES, (TR::SPLIT && p) ? &tm_v_lo : &tm_v, &kv_full[s], col(p), j * BN, it.hd, it.bt);
                 }
+                idx = item_take(source, n, pp.n_items, ab);
+                item_ring_publish(ring, n, idx, ab);
             }
             pdl_trigger();      // this CTA's last loads are out: the next kernel may start as the SMs empty (triggered at the start instead, the next
                                 // kernel's waiting CTAs cost the backward 5-10 %)

@@ -228,7 +228,12 @@ struct ItemRing {
 __device__ __forceinline__ void item_ring_init(const ItemRing& r, uint32_t readers) {
     for (int s = 0; s < 2; ++s) { mbar_init(&r.full[s], 1); mbar_init(&r.empty[s], readers); }
 }
-// Producer thread: ask for the next item (the answer is needed only after the current item's first loads), and take it.
+// Producer thread: ask for the next item with the last loads of the current one, and take it after them.  The roles behind it
+// still have the ring's depth of tiles ahead, which hides the answer (asking 2, 5 or 12 tiles earlier changed nothing), and an item
+// goes to the CTA that is about to run out.  Asked for with an item's first loads, the second item of every CTA was claimed while
+// the first ones, the longest walks, had only begun, and so some CTAs got two long ones: forward of 16 heads T = 4096 D = 128
+// 81 us, now 60; forward and backward of 96 fp32 heads T = 1024 75.8 and 172 us, now 73.5 and 168; backward of 32 heads T = 8192
+// 1549 us, now 1516.
 struct ItemSource {
     uint4* response;       // 16-byte aligned shared memory
     uint64_t* bar;         // count 1
