@@ -210,7 +210,8 @@ int ib200_cast_bf16_to_f32(const void* src, float* dst, size_t n, ib200_stream_t
  * `sm_count` SMs.  Item i of the list is unit `units[i]` (forward: pair of 128-row query tiles, backward: 128-row key tile) of
  * head `heads[i]` (0 <= head < B*H); units are numbered as the tensor is (unit 0 = first rows).  The list runs over groups of
  * consecutive heads; `*n_groups` receives their number.  At most `capacity` entries are written; the return value is the
- * number of items of the list, or a negative IB200_ERR_* value.  The reference has no counterpart (it launches one thread
+ * number of items of the list, or a negative IB200_ERR_* value.  A forward too small to fill the SMs walks single query
+ * tiles instead of pairs, in a list of the same form.  The reference has no counterpart (it launches one thread
  * per score row, src/inferno/cuda/cudasoftmax.cu:52-97). */
 int ib200_attn_item_order(int pass, int B, int H, int T, int D, int sm_count, int* heads, int* units, int capacity, int* n_groups);
 

@@ -181,13 +181,13 @@ int persist_head_groups(int ctas, int items_per_head, long BH, size_t shared_byt
     return static_cast<int>(n_groups < 1 ? 1 : n_groups);
 }
 
-// Persistent CTAs walking (head, query-tile pair) items, heaviest first.  SPLIT: fp32 I/O, operands given as dense
+// Persistent CTAs walking (head, query-tile pair) items, or with ONE_TILE (head, query tile) items, heaviest first.  SPLIT: fp32 I/O, operands given as dense
 // (hi, lo) bf16 copies (q_lo, k_lo, v_lo), output fp32.
-template <int D, bool SPLIT>
-int launch_fwd_persist(const void* q, const void* q_lo, const void* k, const void* k_lo, const void* v, const void* v_lo, void* o,
+template <int D, bool SPLIT, bool ONE_TILE>
+int launch_fwd_items(const void* q, const void* q_lo, const void* k, const void* k_lo, const void* v, const void* v_lo, void* o,
                        const RowLayout& lq, const RowLayout& lk, const RowLayout& lv, const RowLayout& lo, float* lse, int* status,
                        long BH, int T, float scale, int causal, cudaStream_t stream) {
-    using TR = FwdPersistTraits<D, SPLIT>;
+    using TR = FwdPersistTraits<D, SPLIT, ONE_TILE>;
     CUtensorMap tq, tql, tk, tkl, tv, tvl, to;
     if (!make_tmap(&tq, q, false, D, T, lq, BH, 128) || !make_tmap(&tk, k, false, D, T, lk, BH, 128) ||
         !make_tmap(&tv, v, false, D, T, lv, BH, 128) || !make_tmap(&to, o, SPLIT, D, T, lo, BH, 128))
@@ -209,17 +209,49 @@ int launch_fwd_persist(const void* q, const void* q_lo, const void* k, const voi
     pp.p.H = lq.H;
     pp.p.causal = causal;
     pp.p.scale_log2 = scale * 1.4426950408889634f;
-    pp.pairs_per_head = (T + 255) / 256;
-    const long items = static_cast<long>(pp.pairs_per_head) * BH;
+    pp.units_per_head = (T + TR::BM_ITEM - 1) / TR::BM_ITEM;
+    const long items = static_cast<long>(pp.units_per_head) * BH;
     if (items > 0x7fffffffL) return IB200_ERR_UNSUPPORTED;
     pp.n_items = static_cast<int>(items);
     const int sms = dev->sms;
-    pp.n_groups = persist_head_groups(sms, pp.pairs_per_head, BH, static_cast<size_t>(T) * D * (SPLIT ? 8 : 4) /*K, V*/);
+    pp.n_groups = persist_head_groups(sms, pp.units_per_head, BH, static_cast<size_t>(T) * D * (SPLIT ? 8 : 4) /*K, V*/);
     IB200_SET_BOUNDS(D, T, lq.H, static_cast<int>(BH / lq.H), static_cast<int>(BH), 0, TR::TM_COLS, status, stream);
     record_timing_event(0, stream);
     const int rc = launch_pdl<attn_fwd_persist_kernel<TR>>(pp.n_items, TR::THREADS, TR::SMEM_BYTES, stream, tq, tql, tk, tkl, tv, tvl, to, pp);
     record_timing_event(1, stream);
     return rc;
+}
+
+// Items of two query tiles (256 rows) or of one, whose key tiles the two softmax groups share.  A pair walks n key tiles in n
+// steps; a single tile walks them in n / 2, but loads each K / V tile for half as many rows, and there are twice as many items
+// to start and finish.  So a list that leaves SMs idle, or is bound by its longest walk, is better cut into single tiles, and a long list
+// into pairs.  The estimate: the longest item or the average load of an SM, whichever is more, in steps of about 1.7 us (D = 128),
+// an item's start and end counting as 2.4 and the second tile's K / V traffic as a tenth.  Pairs against single tiles, us:
+//   B x H, T, D             pairs  single        B x H, T, D             pairs  single
+//   12, 200, 64               7.7     6.2        16, 4096, 128             60      68
+//   15, 777, 128             16.0    12.3        32, 4096, 128            120     136
+//   4, 4096, 128             57.0    33.5        48, 1024, 64            18.9    22.3
+//   8, 4096, 128             58.3    35.7        64, 512, 128            14.3    16.6
+//   12, 4096, 128            59.7    54.0        24, 1024, 64 fp32       30.9    24.7
+bool fwd_one_tile(long BH, int T, int causal, int sms) {
+    const double n = (T + 127) / 128, p = (T + 255) / 256;       // key tiles = query tiles; pairs
+    const bool odd = 2 * p > n;
+    const double c = 2.4;
+    // steps of all items of a head
+    const double pair_steps = causal ? p * (p + 1) - (odd ? 1 : 0) : p * n;
+    const double one_steps = causal ? (odd ? p * p : p * (p + 1)) : n * p;
+    const double pairs = std::max(n + c, BH * (pair_steps + c * p) / sms), ones = 1.1 * std::max(p + c, BH * (one_steps + c * n) / sms);
+    return ones < pairs;
+}
+
+template <int D, bool SPLIT>
+int launch_fwd_persist(const void* q, const void* q_lo, const void* k, const void* k_lo, const void* v, const void* v_lo, void* o,
+                       const RowLayout& lq, const RowLayout& lk, const RowLayout& lv, const RowLayout& lo, float* lse, int* status,
+                       long BH, int T, float scale, int causal, cudaStream_t stream) {
+    const DeviceInfo* dev = device_info();
+    if (!dev) return IB200_ERR_CUDA;
+    auto launch = fwd_one_tile(BH, T, causal, dev->sms) ? launch_fwd_items<D, SPLIT, true> : launch_fwd_items<D, SPLIT, false>;
+    return launch(q, q_lo, k, k_lo, v, v_lo, o, lq, lk, lv, lo, lse, status, BH, T, scale, causal, stream);
 }
 
 // Persistent CTAs walking (head, key tile) items, longest walks first.  SPLIT (fp32 I/O): every operand is given as dense

@@ -11,6 +11,8 @@
 // A CTA launched per item pays about 7 us for launch, the first loads, the pipeline fill and the epilogue (measured on
 // the one-CTA-per-item form this kernel replaced): 20 % of an average item at T = 4096 and half of one at T = 1024;
 // here most of it runs under another item's work.
+// A list too short to fill the SMs, or bound by its longest walk, is cut into single query tiles instead (ONE_TILE; the host
+// decides): the two softmax groups then take the tile's key tiles in turn, so the walk has half as many steps.
 // All mbarrier phases run on from item to item; each role derives them from its own counters.
 // Items are drawn, not assigned: a CTA starts on item blockIdx.x and its TMA thread takes over the items of CTAs that have not
 // been launched yet (ItemRing in sm100_ptx.cuh hands them to the other roles), so CTAs that drew short walks draw more
@@ -22,9 +24,16 @@
 
 namespace ib200 {
 
-template <int D_, bool SPLIT_ = false>
+// ONE_TILE: an item is one query tile, and the two softmax groups take its key tiles in turn (group 0 the even ones, group 1
+// the odd ones), each with its own S, O, maximum and sum; the epilogue puts the two halves together.
+template <int D_, bool SPLIT_ = false, bool ONE_TILE_ = false>
 struct FwdPersistTraits : FwdTraits<D_, SPLIT_> {
     using Base = FwdTraits<D_, SPLIT_>;
+    static constexpr bool ONE_TILE = ONE_TILE_;
+    static constexpr int BM_ITEM = ONE_TILE ? 128 : 256;
+    // ONE_TILE: each group writes one 128-byte panel of the output; where there is only one, group 0 writes it
+    static constexpr bool BOTH_WRITE = ONE_TILE && Base::OUT_PANELS == 2;
+    static constexpr int OFF_EXCHANGE = Base::TILE_BYTES;                      // ONE_TILE: the groups' maxima and sums, in the second query tile's place
     static constexpr int OFF_STAGE = Base::SMEM_TILES * Base::TILE_BYTES;      // one O staging tile, used by both query tiles in turn
     static constexpr int OFF_BAR = OFF_STAGE + Base::TILE_BYTES;
     static constexpr int SMEM_BYTES = OFF_BAR + 512 + 1024 /*align slack*/;
@@ -33,8 +42,8 @@ struct FwdPersistTraits : FwdTraits<D_, SPLIT_> {
 
 struct FwdPersistParams {
     FwdParams p;
-    int n_items;        // pairs_per_head * BH
-    int pairs_per_head; // ceil(T / 256)
+    int n_items;        // units_per_head * BH
+    int units_per_head; // ceil(T / BM_ITEM)
     int n_groups;       // head groups of the item list (see locate_item)
 };
 
@@ -65,7 +74,8 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     uint64_t* stage_free = o_free + 2;      // [1]   the TMA store has read the staging tile
     uint64_t* ring_bars = stage_free + 1;   // [4]   item ring: full[2], empty[2]
     uint64_t* clc_bar = ring_bars + 4;      // [1]   answer to the request for another item
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ring_bars + 5);
+    uint64_t* half_full = clc_bar + 1;      // [2]   ONE_TILE: group i's maxima and sums of an item are in shared memory (4 warps)
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(half_full + 2);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     const ItemRing ring{ring_bars, ring_bars + 2, abort_flag + 1};
     const ItemSource source{reinterpret_cast<uint4*>(smem + TR::OFF_BAR + 496), clc_bar};
@@ -74,17 +84,26 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     const int T = prm.T;
     const int BH = prm.BH;
     const int n_kv_total = (T + BN - 1) / BN;
+    constexpr int kAhead = TR::ONE_TILE ? 2 : 1;            // load group j brings V_j and K_{j + kAhead}
     AbortCtx ab{abort_flag, prm.status};
 
     // item -> head, query tiles, key-tile counts (identical in every role)
+    // nkv: key tiles of each softmax group; n_iter: key tiles loaded
     struct Item { int bh, hd, bt, m0, m1, nkv0, nkv1, n_iter; };
     auto decode = [&](int idx) {
         Item it;
         int rank;
-        locate_item(HeadGroups{BH, pp.n_groups, pp.pairs_per_head}, idx, rank, it.bh);
-        const int pair = pp.pairs_per_head - 1 - rank;            // the last pair walks the most key tiles: first
+        locate_item(HeadGroups{BH, pp.n_groups, pp.units_per_head}, idx, rank, it.bh);
+        const int pair = pp.units_per_head - 1 - rank;            // the last pair (tile) walks the most key tiles: first
         it.hd = it.bh % prm.H;
         it.bt = it.bh / prm.H;
+        if constexpr (TR::ONE_TILE) {
+            it.m0 = it.m1 = pair;
+            it.n_iter = prm.causal ? min(pair + 1, n_kv_total) : n_kv_total;
+            it.nkv0 = (it.n_iter + 1) >> 1;
+            it.nkv1 = it.n_iter >> 1;
+            return it;
+        }
         it.m0 = 2 * pair;
         it.m1 = 2 * pair + 1;
         const bool v0 = it.m0 * BM < T, v1 = it.m1 * BM < T;
@@ -102,7 +121,8 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
         for (int s = 0; s < KS; ++s) { mbar_init(&kv_full[s], 1); mbar_init(&kv_empty[s], 1); }
         for (int i = 0; i < 2; ++i) {
             mbar_init(&s_full[i], 1); mbar_init(&p_half[2 * i], 4); mbar_init(&p_half[2 * i + 1], 4);
-            mbar_init(&o_full[i], 1); mbar_init(&o_free[i], 4);
+            mbar_init(&o_full[i], 1); mbar_init(&o_free[i], TR::BOTH_WRITE ? 8 : 4);
+            mbar_init(&half_full[i], 4);
         }
         mbar_init(stage_free, 1);
         mbar_init(clc_bar, 1);
@@ -132,27 +152,31 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                 if (*abort_flag != 0) break;
                 const Item it = decode(idx);
                 if (n > 0) mbar_wait(q_free, (n - 1) & 1, ab, 12);
-                const int q_tiles = (it.nkv1 > 0) ? 2 : 1;
-                mbar_arrive_expect_tx(q_full, (q_tiles + 1) * TR::TILE_BYTES);
+                const int q_tiles = (!TR::ONE_TILE && it.nkv1 > 0) ? 2 : 1;
+                const int k_tiles = (TR::ONE_TILE && it.n_iter > 1) ? 2 : 1;      // key tiles loaded ahead of the first P.V
+                mbar_arrive_expect_tx(q_full, (q_tiles + k_tiles) * TR::TILE_BYTES);
                 // panel p of a tile: columns 64p.. of a bf16 operand, or (fp32 I/O) the hi / lo half of the bf16 pair
                 auto col = [](int p) { return TR::SPLIT ? 0 : p * 64; };
                 for (int p = 0; p < TR::NP; ++p) tma_load_4d(sQ + p * TR::PANEL_BYTES, (TR::SPLIT && p) ? &tm_q_lo : &tm_q, q_full, col(p), it.m0 * BM, it.hd, it.bt);
                 if (q_tiles == 2)
                     for (int p = 0; p < TR::NP; ++p)
                         tma_load_4d(sQ + TR::TILE_BYTES + p * TR::PANEL_BYTES, (TR::SPLIT && p) ? &tm_q_lo : &tm_q, q_full, col(p), it.m1 * BM, it.hd, it.bt);
-                for (int p = 0; p < TR::NP; ++p)
-                    tma_load_4d(sK + (G % KS) * TR::TILE_BYTES + p * TR::PANEL_BYTES, (TR::SPLIT && p) ? &tm_k_lo : &tm_k, q_full, col(p), 0, it.hd, it.bt);
+                for (int j = 0; j < k_tiles; ++j)
+                    for (int p = 0; p < TR::NP; ++p)
+                        tma_load_4d(sK + ((G + j) % KS) * TR::TILE_BYTES + p * TR::PANEL_BYTES, (TR::SPLIT && p) ? &tm_k_lo : &tm_k, q_full, col(p), j * BN, it.hd,
+                                    it.bt);
                 for (int j = 0; j < it.n_iter; ++j, ++G) {
                     const int s = G % KS;
-                    const bool has_k = (j + 1) < it.n_iter;
+                    const bool has_k = (j + kAhead) < it.n_iter;
                     mbar_wait(&kv_empty[s], ((G / KS) & 1) ^ 1, ab, 10);
-                    if (!has_k) item_request(source);        // KS key tiles before the item's end (see ItemSource)
-                    if (j == KS - 1) mbar_wait(k0_free, n & 1, ab, 11);         // K_KS reuses the slot of K_0
+                    if (j + 1 == it.n_iter) item_request(source);        // KS key tiles before the item's end (see ItemSource)
+                    // K_KS reuses the slot of K_0 (ONE_TILE: and K_KS+1 that of K_1, which k0_free covers too)
+                    if (j == KS - kAhead && (kAhead == 1 || has_k)) mbar_wait(k0_free, n & 1, ab, 11);
                     mbar_arrive_expect_tx(&kv_full[s], (has_k ? 2 : 1) * TR::TILE_BYTES);
                     if (has_k)
                         for (int p = 0; p < TR::NP; ++p)
-                            tma_load_4d(sK + ((G + 1) % KS) * TR::TILE_BYTES + p * TR::PANEL_BYTES, (TR::SPLIT && p) ? &tm_k_lo : &tm_k, &kv_full[s], col(p),
-                                        (j + 1) * BN, it.hd, it.bt);
+                            tma_load_4d(sK + ((G + kAhead) % KS) * TR::TILE_BYTES + p * TR::PANEL_BYTES, (TR::SPLIT && p) ? &tm_k_lo : &tm_k, &kv_full[s], col(p),
+                                        (j + kAhead) * BN, it.hd, it.bt);
                     for (int p = 0; p < TR::NP; ++p)
                         tma_load_4d(sV + s * TR::TILE_BYTES + p * TR::PANEL_BYTES, (TR::SPLIT && p) ? &tm_v_lo : &tm_v, &kv_full[s], col(p), j * BN, it.hd, it.bt);
                 }
@@ -181,36 +205,37 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
 #pragma unroll
             for (int i = 0; i < 2; ++i)
                 if (nkv[i] > 0) {
-                    fwd_issue_s<TR>(tmem + (i ? TR::TM_S1 : TR::TM_S0), q_lo[i], k_lo0 + (G % KS) * kStage, leader);
+                    fwd_issue_s<TR>(tmem + (i ? TR::TM_S1 : TR::TM_S0), q_lo[TR::ONE_TILE ? 0 : i], k_lo0 + ((G + (TR::ONE_TILE ? i : 0)) % KS) * kStage, leader);
                     if (leader) umma_commit(&s_full[i]);
                 }
             if (leader) umma_commit(k0_free);
-            if (it.n_iter == 1 && leader) umma_commit(q_free);
+            if (it.n_iter <= kAhead && leader) umma_commit(q_free);
             for (int j = 0; j < it.n_iter; ++j, ++G) {
                 const int sv = G % KS;
-                const uint32_t v_lo = v_lo0 + sv * kStage, k_next_lo = k_lo0 + ((G + 1) % KS) * kStage;
+                const uint32_t v_lo = v_lo0 + sv * kStage, k_next_lo = k_lo0 + ((G + kAhead) % KS) * kStage;
                 mbar_wait(&kv_full[sv], (G / KS) & 1, ab, 22);
 #pragma unroll
                 for (int i = 0; i < 2; ++i) {
-                    if (j < nkv[i]) {
+                    const int jj = TR::ONE_TILE ? j >> 1 : j;              // key tile of this group
+                    if (TR::ONE_TILE ? (j & 1) == i : j < nkv[i]) {
                         const uint32_t tm_s = tmem + (i ? TR::TM_S1 : TR::TM_S0), tm_o = tmem + (i ? TR::TM_O1 : TR::TM_O0);
                         // the first P.V of an item overwrites O_i: the previous item's epilogue must have read it
-                        if (j == 0 && oc[i] > 0) mbar_wait(&o_free[i], (oc[i] - 1) & 1, ab, 26);
+                        if (jj == 0 && oc[i] > 0) mbar_wait(&o_free[i], (oc[i] - 1) & 1, ab, 26);
                         mbar_wait(&p_half[2 * i], pc[i] & 1, ab, 24);
                         tc_fence_after_sync();
                         if constexpr (!TR::SPLIT) {
-                            fwd_issue_pv_part<TR, 0, TR::PV_KSTEPS / 2>(tm_o, tm_s, v_lo, j == 0, leader);
+                            fwd_issue_pv_part<TR, 0, TR::PV_KSTEPS / 2>(tm_o, tm_s, v_lo, jj == 0, leader);
                             mbar_wait(&p_half[2 * i + 1], pc[i] & 1, ab, 25);
                             tc_fence_after_sync();
-                            fwd_issue_pv_part<TR, TR::PV_KSTEPS / 2, TR::PV_KSTEPS>(tm_o, tm_s, v_lo, j == 0, leader);
+                            fwd_issue_pv_part<TR, TR::PV_KSTEPS / 2, TR::PV_KSTEPS>(tm_o, tm_s, v_lo, jj == 0, leader);
                         } else {
                             mbar_wait(&p_half[2 * i + 1], pc[i] & 1, ab, 25);
                             tc_fence_after_sync();
-                            fwd_issue_pv<TR>(tm_o, tm_s, v_lo, j == 0, leader);
+                            fwd_issue_pv<TR>(tm_o, tm_s, v_lo, jj == 0, leader);
                         }
                         ++pc[i];
-                        if (j + 1 < nkv[i]) {
-                            fwd_issue_s<TR>(tm_s, q_lo[i], k_next_lo, leader);
+                        if (jj + 1 < nkv[i]) {
+                            fwd_issue_s<TR>(tm_s, q_lo[TR::ONE_TILE ? 0 : i], k_next_lo, leader);
                             if (leader) umma_commit(&s_full[i]);
                         } else {
                             if (leader) umma_commit(&o_full[i]);           // last key tile of this query tile: O_i is final
@@ -219,8 +244,8 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                     }
                 }
                 if (leader) umma_commit(&kv_empty[sv]);
-                // the item's last S MMAs were issued in iteration n_iter - 2: Q and the K slots are free once they complete
-                if (j == it.n_iter - 2 && leader) umma_commit(q_free);
+                // the item's last S MMAs were issued in iteration n_iter - 1 - kAhead: Q and the K slots are free once they complete
+                if (j == it.n_iter - 1 - kAhead && leader) umma_commit(q_free);
             }
         }
     } else if (warp < 8) {
@@ -235,6 +260,7 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
         const float c = prm.scale_log2;
         uint32_t sc = 0;                         // S tiles consumed so far (phase of s_full)
         uint32_t oc = 0;                         // items in which this query tile was valid (phase of o_full)
+        uint32_t n2 = 0;                         // ONE_TILE: items with two halves
         int n = 0;
         for (int idx = blockIdx.x; idx < pp.n_items; idx = item_ring_next(ring, n++, ab, lane == 0)) {
             if (*abort_flag != 0) break;
@@ -257,8 +283,9 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                 }
                 tmem_wait_ld();
                 // masking: causal on the diagonal tile; keys past T on the last tile
-                const int col0 = j * BN;
-                const bool diag = prm.causal && (j == m_tile);
+                const int key_tile = TR::ONE_TILE ? 2 * j + i : j;
+                const int col0 = key_tile * BN;
+                const bool diag = prm.causal && (key_tile == m_tile);
                 const bool tail = (col0 + BN > T);
                 if (diag || tail) {
                     const int limit = diag ? min(row_g, T - 1) : (T - 1);   // last visible key
@@ -337,6 +364,101 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                 if (lane == 0) mbar_arrive(&p_half[2 * i + 1]);
             }
 
+            if constexpr (TR::ONE_TILE) {
+                // ---- epilogue of the item: O = (wa O_0 + wb O_1) / (wa l_0 + wb l_1), w = 2^(m - max) ----
+                // A group publishes its row's (m, l) only after its own O is final, i.e. after both groups have read the previous
+                // item's O and with it the previous item's (m, l); group 1 takes no part in the exchange when the item has one key tile.
+                const bool two = it.nkv1 > 0;
+                float2* exchange = reinterpret_cast<float2*>(smem + TR::OFF_EXCHANGE);
+                const int writer_groups = TR::BOTH_WRITE ? 2 : 1;
+                if (i == 0 || two) {
+                    mbar_wait(&o_full[i], oc & 1, ab, 32);
+                    if (i == 0 ? TR::BOTH_WRITE : true) {
+                        exchange[i * 128 + t] = make_float2(m_used, l);
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&half_full[i]);
+                    }
+                    ++oc;
+                }
+                if (i < writer_groups) {
+                    // this group's view: (m0, l0) of the even tiles, (m1, l1) of the odd ones
+                    float m0 = m_used, l0 = l, m1 = 0.f, l1 = 0.f;
+                    if (i == 1) {
+                        mbar_wait(&half_full[0], n & 1, ab, 35);
+                        const float2 x = exchange[t];
+                        m1 = m_used; l1 = two ? l : 0.f;
+                        m0 = x.x; l0 = x.y;
+                    } else if (two) {
+                        mbar_wait(&half_full[1], n2 & 1, ab, 36);
+                        const float2 x = exchange[128 + t];
+                        m1 = x.x; l1 = x.y;
+                    }
+                    if (two) ++n2;
+                    if (i == 1) mbar_wait(&o_full[0], n & 1, ab, 37);
+                    else if (two) mbar_wait(&o_full[1], (n2 - 1) & 1, ab, 38);
+                    tc_fence_after_sync();
+                    // a half without any weight (every score -inf) must not set the reference point; a NaN sum still counts
+                    if (l0 == 0.f) m0 = m1;
+                    if (l1 == 0.f) m1 = m0;
+                    const float mm = fmaxf(m0, m1);
+                    const float w0 = fast_exp2(m0 - mm), w1 = fast_exp2(m1 - mm);
+                    const float ll = w0 * l0 + w1 * l1;
+                    const float f0 = w0 / ll, f1 = w1 / ll;
+                    const uint32_t t0 = tmem + TR::TM_O0 + lane_base, t1 = tmem + TR::TM_O1 + lane_base;
+                    constexpr int kCols = TR::BOTH_WRITE ? D / 2 : D;
+                    const int c0 = TR::BOTH_WRITE ? i * kCols : 0;
+                    uint8_t* panel = sO + (TR::BOTH_WRITE ? i * TR::PANEL_BYTES : 0);
+                    if (n > 0) {
+                        if (t == 0) tma_store_wait_read_all();       // this group's previous store has read its panel
+                        asm volatile("bar.sync %0, 128;" ::"r"(1 + i) : "memory");
+                    }
+#pragma unroll
+                    for (int cc = 0; cc < kCols; cc += 32) {
+                        uint32_t r[32];
+                        float o[32];
+                        tmem_ld_x32(t0 + c0 + cc, r);
+                        tmem_wait_ld();
+#pragma unroll
+                        for (int e = 0; e < 32; ++e) o[e] = __uint_as_float(r[e]) * f0;
+                        if (two) {
+                            tmem_ld_x32(t1 + c0 + cc, r);
+                            tmem_wait_ld();
+#pragma unroll
+                            for (int e = 0; e < 32; ++e) o[e] = fmaf(__uint_as_float(r[e]), f1, o[e]);
+                        }
+                        if (cc + 32 == kCols) {
+                            // both halves are in registers: the next item's first P.V may overwrite them
+                            tc_fence_before_sync();
+                            __syncwarp();
+                            if (lane == 0) {
+                                mbar_arrive(&o_free[0]);
+                                if (two) mbar_arrive(&o_free[1]);
+                            }
+                        }
+                        if constexpr (!TR::SPLIT) {
+#pragma unroll
+                            for (int q4 = 0; q4 < 4; ++q4)
+                                st_shared_sw128(panel, t, (cc / 8 + q4) & 7,
+                                                make_uint4(pack_bf16x2(o[q4 * 8], o[q4 * 8 + 1]), pack_bf16x2(o[q4 * 8 + 2], o[q4 * 8 + 3]),
+                                                           pack_bf16x2(o[q4 * 8 + 4], o[q4 * 8 + 5]), pack_bf16x2(o[q4 * 8 + 6], o[q4 * 8 + 7])));
+                        } else {
+#pragma unroll
+                            for (int q4 = 0; q4 < 8; ++q4)
+                                st_shared_sw128(panel, t, q4,
+                                                make_uint4(__float_as_uint(o[q4 * 4]), __float_as_uint(o[q4 * 4 + 1]), __float_as_uint(o[q4 * 4 + 2]),
+                                                           __float_as_uint(o[q4 * 4 + 3])));
+                        }
+                    }
+                    if (i == 0 && row_g < T) prm.lse[static_cast<size_t>(it.bh) * T + row_g] = (mm + log2f(ll)) * 0.6931471805599453f;
+                    fence_proxy_async_smem();
+                    asm volatile("bar.sync %0, 128;" ::"r"(1 + i) : "memory");
+                    if (t == 0) {
+                        tma_store_4d(&tm_o, panel, TR::BOTH_WRITE ? i * TR::OUT_PANEL_ELEMS : 0, m_tile * BM, it.hd, it.bt);
+                        tma_store_commit();
+                    }
+                }
+                continue;
+            }
             // ---- epilogue of this query tile; the staging tile is used by tile 0 and tile 1 of every item in turn ----
             const uint32_t use = 2u * static_cast<uint32_t>(n) + static_cast<uint32_t>(i);
             if (nkv > 0) {
@@ -400,6 +522,7 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
         }
     }
 
+    if (TR::ONE_TILE && (tid & 127) == 0 && warp < 8) tma_store_wait_read_all();
     // ------------------------------ tear-down ------------------------------
     tc_fence_before_sync();
     __syncthreads();

@@ -281,3 +281,63 @@ def test_abi_errors_on_gpu():
     import ctypes
     code = ctypes.c_int(-1)
     assert L.ib200_attn_check(ws.data_ptr(), s, ctypes.byref(code)) == _capi.OK and code.value == 0
+
+
+def _eval64(q, k, v, causal):
+    """O and lse in 64 bits on the GPU."""
+    q, k, v = (t.double() for t in (q, k, v))
+    s = q @ k.transpose(-1, -2) / q.shape[-1] ** 0.5
+    if causal:
+        s = s.masked_fill(torch.ones(s.shape[-2:], dtype=torch.bool, device=s.device).triu(1), float("-inf"))
+    return torch.softmax(s, -1) @ v, torch.logsumexp(s, -1)
+
+
+# One head leaves SMs idle: its query tiles are separate items and two softmax groups share a tile's keys.  148 x 4 copies of it
+# are walked in pairs of tiles.  One to ten key tiles (odd and even, past the ring of two or four), a last tile of one row, exact tiles.
+@pytest.mark.parametrize("T", [128, 129, 255, 257, 384, 513, 640, 1161])
+@pytest.mark.parametrize("dt,D", [("bf16", 64), ("bf16", 128), ("f32", 64)])
+@pytest.mark.parametrize("causal", [True, False])
+def test_single_tile_items_and_tile_pairs_agree(T, dt, D, causal):
+    q, k, v = (torch.from_numpy(a).cuda().to(TDT[dt]) for a in make_inputs(1, 1, T, D, 300 + T, 1.5, 1.0, dt)[:3])
+    ref, lse_ref = _eval64(q, k, v, causal)
+    many = [t.expand(148, 4, T, D).contiguous() for t in (q, k, v)]
+    runs = [A.attention_forward(q, k, v, causal=causal), A.attention_forward(*many, causal=causal)]
+    torch.cuda.synchronize()
+    A.check_device_status()
+    # bf16: P and O are rounded to 8 bits (2^-9 each); fp32: operands and P as bf16 pairs, 2^-16 each, three factors
+    tol = 2 * 2.0 ** -8 if dt == "bf16" else 3 * 2.0 ** -16
+    for o, lse in runs:
+        assert ((o.double() - ref).norm(dim=(-1, -2)) / ref.norm()).max() < tol
+        assert (lse.double() - lse_ref).abs().max() < 1e-4
+    # a CTA's items follow one another in both: every copy is the same, bit for bit
+    assert torch.equal(runs[1][0], runs[1][0][:1, :1].expand_as(runs[1][0]))
+
+
+# More single-tile items than SMs: barriers run on from item to item, with one key tile and with many.
+@pytest.mark.parametrize("B,H,T,D,dt", [(2, 12, 1024, 64, "f32"), (1, 12, 4096, 128, "bf16"), (1, 8, 4000, 64, "bf16")])
+def test_single_tile_items_in_several_rounds(B, H, T, D, dt):
+    one = [torch.from_numpy(a).cuda().to(TDT[dt]) for a in make_inputs(1, 1, T, D, 41, 1.0, 1.0, dt)[:3]]
+    ref, lse_ref = _eval64(*one, True)
+    o, lse = A.attention_forward(*(t.expand(B, H, T, D).contiguous() for t in one))
+    torch.cuda.synchronize()
+    A.check_device_status()
+    tol = 2 * 2.0 ** -8 if dt == "bf16" else 3 * 2.0 ** -16
+    assert torch.equal(o, o[:1, :1].expand_as(o)) and torch.equal(lse, lse[:1, :1].expand_as(lse))
+    assert (o[0, 0].double() - ref[0, 0]).norm() / ref.norm() < tol and (lse[0, 0].double() - lse_ref[0, 0]).abs().max() < 1e-4
+
+
+def test_single_tile_items_keep_infinities():
+    """A half whose scores are all -inf has no weight; a NaN score reaches its row and no other (as with tile pairs)."""
+    q, k, v = (torch.from_numpy(a).cuda().to(torch.bfloat16) for a in make_inputs(1, 1, 512, 128, 9, 1.0, 1.0, "bf16")[:3])
+    q[..., 0] = q[..., 0].abs() + 0.5
+    k[:, :, 128:256, 0] = float("-inf")             # the second key tile: all of the odd half's keys for rows 128..383
+    q[:, :, 500, 3] = float("nan")
+    many = [t.expand(148, 4, 512, 128).contiguous() for t in (q, k, v)]
+    o, lse = A.attention_forward(q, k, v)
+    o2, lse2 = A.attention_forward(*many)
+    ref, lse_ref = _eval64(q, k, v, True)
+    A.check_device_status()
+    for x, l in ((o[0, 0], lse[0, 0]), (o2[0, 0], lse2[0, 0])):
+        assert torch.equal(torch.isnan(x), torch.isnan(ref[0, 0])) and torch.equal(torch.isnan(l), torch.isnan(lse_ref[0, 0]))
+        ok = ~torch.isnan(lse_ref[0, 0])
+        assert (x[ok].double() - ref[0, 0][ok]).norm() / ref[0, 0][ok].norm() < 2 * 2.0 ** -8
