@@ -7,7 +7,8 @@ Here the same round trip is chunked over heads and pipelined on three streams --
 copies, kernels, device-to-host copies -- with double-buffered device staging, so that the copies
 of one chunk overlap the kernels of another.  A staging set's input half is released as soon as the
 kernels have consumed it and its output half once the results have left, so neither copy direction
-ever waits for the other.  Heads are independent, so chunking changes nothing.
+ever waits for the other.  Heads are independent: chunking changes at most
+the rounding of O, where the forward cuts the list of a chunk differently from that of all heads.
 """
 from __future__ import annotations
 
