@@ -247,18 +247,23 @@ Grads attention_backward(const Tensor& q_, const Tensor& k_, const Tensor& v_, c
 }
 
 // ---- autograd nodes ----------------------------------------------------------------
+// The ops have no forward-mode derivative: a dual input must not lose its tangent silently.
+void refuse_tangents(std::initializer_list<const Tensor*> ts, const char* op) {
+    for (const Tensor* t : ts)
+        TORCH_CHECK_NOT_IMPLEMENTED(!t->defined() || !t->_fw_grad(0).defined(), op, ": forward-mode differentiation is not implemented");
+}
+
 // The backward node of the fused op: saves q, k, v, out and lse; produces dq, dk, dv.  Plays the role a
 // `class AttentionBackward : public Node` has in the reference (src/inferno/gradfn/node.h:23-45).
 struct AttentionBackward : torch::autograd::Node {
-    SavedVariable q, k, v, o;
-    Tensor lse;
+    SavedVariable q, k, v, o, lse;
     double scale = 0;
     bool causal = true;
     int math_mode = 0;
 
     variable_list apply(variable_list&& grads) override {
         if (!grads[0].defined()) return variable_list(3);
-        const Tensor tq = q.unpack(), tk = k.unpack(), tv = v.unpack(), to = o.unpack(shared_from_this());
+        const Tensor tq = q.unpack(), tk = k.unpack(), tv = v.unpack(), to = o.unpack(shared_from_this()), tl = lse.unpack();
         at::AutoDispatchBelowADInplaceOrView below;
         const int64_t B = tq.size(0), H = tq.size(1), T = tq.size(2), D = tq.size(3), step = H * D * tq.element_size();
         auto at_byte = [](const Tensor& t) { return static_cast<const char*>(t.data_ptr()); };
@@ -271,17 +276,17 @@ struct AttentionBackward : torch::autograd::Node {
             dk = g.select(2, 1).transpose(1, 2);
             dv = g.select(2, 2).transpose(1, 2);
         }
-        const Grads r = attention_backward(tq, tk, tv, to, grads[0], lse, scale, causal, math_mode, dq, dk, dv);
+        const Grads r = attention_backward(tq, tk, tv, to, grads[0], tl, scale, causal, math_mode, dq, dk, dv);
         return {r.dq, r.dk, r.dv};
     }
     void release_variables() override {
-        q.reset_data(); k.reset_data(); v.reset_data(); o.reset_data();
-        lse.reset();
+        q.reset_data(); k.reset_data(); v.reset_data(); o.reset_data(); lse.reset_data();
     }
     std::string name() const override { return "AttentionBackward"; }
 };
 
 Tensor causal_attention(const Tensor& q, const Tensor& k, const Tensor& v, const std::optional<double>& scale, bool causal, int math_mode, bool bthd) {
+    refuse_tangents({&q, &k, &v}, "causal_attention");
     const bool differentiable = torch::autograd::compute_requires_grad(q, k, v);
     Tensor o, lse;
     {
@@ -294,7 +299,7 @@ Tensor causal_attention(const Tensor& q, const Tensor& k, const Tensor& v, const
         node->q = SavedVariable(q, false);
         node->k = SavedVariable(k, false);
         node->v = SavedVariable(v, false);
-        node->lse = lse;
+        node->lse = SavedVariable(lse, false);
         node->scale = scale ? *scale : 1.0 / std::sqrt(static_cast<double>(q.size(3)));
         node->causal = causal;
         node->math_mode = math_mode;
@@ -308,15 +313,14 @@ Tensor causal_attention(const Tensor& q, const Tensor& k, const Tensor& v, const
 // buffer, autograd would fill a zeroed buffer per view, copy each slice's gradient into it and add the three up (240 of the
 // 490 us of a 12-head T = 1024 B = 16 layer); here dq, dk, dv land in their places in the gradient itself.
 struct PackedAttentionBackward : torch::autograd::Node {
-    SavedVariable qkv, o;      // o: [B, T, C]
-    Tensor lse;
+    SavedVariable qkv, o, lse;      // o: [B, T, C]
     int64_t H = 0;
     float scale = 0;
     int math_mode = 0;
 
     variable_list apply(variable_list&& grads) override {
         if (!grads[0].defined()) return variable_list(1);
-        const Tensor p = qkv.unpack(), to = o.unpack(shared_from_this());
+        const Tensor p = qkv.unpack(), to = o.unpack(shared_from_this()), tl = lse.unpack();
         at::AutoDispatchBelowADInplaceOrView below;
         const c10::cuda::CUDAGuard guard(p.device());
         const int64_t B = p.size(0), T = p.size(1), C = p.size(2) / 3, D = C / H;
@@ -329,13 +333,12 @@ struct PackedAttentionBackward : torch::autograd::Node {
             dy = dy.contiguous();
         Tensor g = at::empty({B, T, 3 * C}, p.options());
         launch_bwd(s, packed_operand(p, 0, C, D), packed_operand(p, 1, C, D), packed_operand(p, 2, C, D), packed_operand(to, 0, C, D),
-                   packed_operand(dy, 0, C, D), lse.data_ptr<float>(), packed_operand(g, 0, C, D), packed_operand(g, 1, C, D), packed_operand(g, 2, C, D), scale,
+                   packed_operand(dy, 0, C, D), tl.data_ptr<float>(), packed_operand(g, 0, C, D), packed_operand(g, 1, C, D), packed_operand(g, 2, C, D), scale,
                    true, math_mode, p.device());
         return {g};
     }
     void release_variables() override {
-        qkv.reset_data(); o.reset_data();
-        lse.reset();
+        qkv.reset_data(); o.reset_data(); lse.reset_data();
     }
     std::string name() const override { return "PackedAttentionBackward"; }
 };
@@ -347,6 +350,7 @@ Tensor causal_attention_packed(const Tensor& qkv, int64_t H, const std::optional
     TORCH_CHECK(qkv.is_cuda(), "causal_attention: tensor is not on a CUDA device (there is no CPU path)");
     TORCH_CHECK_TYPE(qkv.scalar_type() == at::kFloat || qkv.scalar_type() == at::kBFloat16,
                      "causal_attention: dtype must be float32 or bfloat16, the same for all tensors");
+    refuse_tangents({&qkv}, "causal_attention");
     const bool differentiable = torch::autograd::compute_requires_grad(qkv);
     Tensor o, lse, p;
     {
@@ -366,7 +370,7 @@ Tensor causal_attention_packed(const Tensor& qkv, int64_t H, const std::optional
         auto node = std::shared_ptr<PackedAttentionBackward>(new PackedAttentionBackward(), torch::autograd::deleteNode);
         node->set_next_edges(torch::autograd::collect_next_edges(qkv));
         node->qkv = SavedVariable(p, false);
-        node->lse = lse;
+        node->lse = SavedVariable(lse, false);
         node->H = H;
         node->scale = scale_of(scale, D);
         node->math_mode = math_mode;
@@ -466,6 +470,7 @@ struct LinearBackward : torch::autograd::Node {
 };
 
 Tensor linear(const Tensor& x, const Tensor& w, const Tensor& bias) {
+    refuse_tangents({&x, &w, &bias}, "linear");
     const bool differentiable = torch::autograd::compute_requires_grad(x, w, bias);
     Tensor y;
     {

@@ -95,3 +95,26 @@ def test_packed_autograd_path_against_the_oracle(oracle_mod, B, H, T, D):
     assert oracle_mod.rel_err(got_y, o) < 2e-2
     for i, ref in enumerate((dq, dk, dv)):
         assert oracle_mod.rel_err(got_g[:, :, i].transpose(0, 2, 1, 3), ref) < 2e-2
+
+
+def test_ops_refuse_tangents_and_save_through_hooks():
+    """A dual input is refused (the ops have no forward-mode derivative), and everything a node keeps passes saved-tensor hooks."""
+    from torch.autograd import forward_ad as fw
+    from inferno_b200.linear import Linear
+    x = torch.randn(1, 2, 64, 64, device="cuda", dtype=torch.bfloat16)
+    qkv = torch.randn(1, 64, 384, device="cuda", dtype=torch.bfloat16)
+    lin = Linear(384, 64).cuda().to(torch.bfloat16)
+    with fw.dual_level():
+        for call in (lambda: A.causal_attention(fw.make_dual(x, x), x, x), lambda: A.causal_attention_packed(fw.make_dual(qkv, qkv), 2),
+                     lambda: lin(fw.make_dual(qkv, qkv))):
+            with pytest.raises(NotImplementedError):
+                call()
+    seen = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: (seen.append(tuple(t.shape)), t)[1], lambda t: t):
+        y = A.causal_attention(x.requires_grad_(), x, x)
+        z = A.causal_attention_packed(qkv.requires_grad_(), 2)
+        want = [(1, 2, 64, 64)] * 4 + [(1, 2, 64)] + [(1, 64, 384), (1, 64, 128), (1, 2, 64)]
+        assert sorted(seen) == sorted(want)
+    torch.autograd.grad((y.float().sum() + z.float().sum()), (x, qkv))
+    torch.cuda.synchronize()
+    A.check_device_status()
