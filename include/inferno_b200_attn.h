@@ -99,6 +99,12 @@ int ib200_attn_fwd_strided(const void* q, const void* k, const void* v, void* o,
                            const ib200_layout* lq, const ib200_layout* lk, const ib200_layout* lv, const ib200_layout* lo,
                            int B, int H, int T, int D, float scale, int causal, int dtype, int math_mode,
                            void* workspace, size_t workspace_bytes, ib200_stream_t stream);
+/* ib200_attn_fwd_strided for a chunk of a larger problem of `total_heads` heads: the walk over the query tiles, which depends on the
+ * number of heads, is the one that a single call on all of them gets, so that chunked and whole results are equal bit for bit. */
+int ib200_attn_fwd_chunk(const void* q, const void* k, const void* v, void* o, float* lse,
+                         const ib200_layout* lq, const ib200_layout* lk, const ib200_layout* lv, const ib200_layout* lo,
+                         int total_heads, int B, int H, int T, int D, float scale, int causal, int dtype, int math_mode,
+                         void* workspace, size_t workspace_bytes, ib200_stream_t stream);
 int ib200_attn_bwd_strided(const void* q, const void* k, const void* v, const void* o, const void* dO, const float* lse,
                            void* dq, void* dk, void* dv,
                            const ib200_layout* lq, const ib200_layout* lk, const ib200_layout* lv, const ib200_layout* lo,

@@ -47,7 +47,7 @@ def attention_forward(q, k, v, scale: float | None = None, causal: bool = True, 
 
     q, k, v (and ``out``) may be arbitrary [B,H,T,D] views with a contiguous last axis -- e.g. slices of a packed
     [B,T,3,H,D] projection, or an output laid out [B,T,H,D] -- and are then read and written in place."""
-    return _capi.host().attention_forward(q, k, v, scale, causal, math_mode, out, lse)
+    return _capi.host().attention_forward(q, k, v, scale, causal, math_mode, out, lse, 0)
 
 
 def attention_backward(q, k, v, o, dO, lse, scale: float | None = None, causal: bool = True,

@@ -247,10 +247,10 @@ bool fwd_one_tile(long BH, int T, int causal, int sms) {
 template <int D, bool SPLIT>
 int launch_fwd_persist(const void* q, const void* q_lo, const void* k, const void* k_lo, const void* v, const void* v_lo, void* o,
                        const RowLayout& lq, const RowLayout& lk, const RowLayout& lv, const RowLayout& lo, float* lse, int* status,
-                       long BH, int T, float scale, int causal, cudaStream_t stream) {
+                       long BH, int T, float scale, int causal, long cut_heads, cudaStream_t stream) {
     const DeviceInfo* dev = device_info();
     if (!dev) return IB200_ERR_CUDA;
-    auto launch = fwd_one_tile(BH, T, causal, dev->sms) ? launch_fwd_items<D, SPLIT, true> : launch_fwd_items<D, SPLIT, false>;
+    auto launch = fwd_one_tile(cut_heads, T, causal, dev->sms) ? launch_fwd_items<D, SPLIT, true> : launch_fwd_items<D, SPLIT, false>;
     return launch(q, q_lo, k, k_lo, v, v_lo, o, lq, lk, lv, lo, lse, status, BH, T, scale, causal, stream);
 }
 
@@ -591,7 +591,7 @@ int linear_bwd_core(const void* x, const void* w, const void* dy, void* dx, void
 
 int fwd_core(const void* q, const void* k, const void* v, void* o, float* lse, const ib200_layout* lq_, const ib200_layout* lk_,
              const ib200_layout* lv_, const ib200_layout* lo_, int B, int H, int T, int D, float scale, int causal, int dtype,
-             int math_mode, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
+             int math_mode, void* workspace, size_t workspace_bytes, long cut_heads /*0: B * H*/, cudaStream_t stream) {
     if (!q || !k || !v || !o || !lse) return IB200_ERR_INVALID_ARGUMENT;
     int rc = check_common(B, H, T, D, dtype, math_mode, causal);
     if (rc != IB200_OK) return rc;
@@ -599,6 +599,8 @@ int fwd_core(const void* q, const void* k, const void* v, void* o, float* lse, c
     if (!aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(o) || !aligned16(lse)) return IB200_ERR_MISALIGNED;
     const long BH = static_cast<long>(B) * H;
     const long N = BH * T * D;
+    if (cut_heads == 0) cut_heads = BH;
+    if (cut_heads < BH) return IB200_ERR_INVALID_ARGUMENT;
     const bool f32 = dtype == IB200_DTYPE_F32;
     RowLayout lq, lk, lv, lo;
     if ((rc = resolve_layout(lq_, H, T, D, f32, &lq)) || (rc = resolve_layout(lk_, H, T, D, f32, &lk)) ||
@@ -630,10 +632,10 @@ int fwd_core(const void* q, const void* k, const void* v, void* o, float* lse, c
         if (rc) return rc;
         const RowLayout dl = dense_layout(H, T, D);
         return launch_fwd_persist<64, true>(part[0], part[1], part[2], part[3], part[4], part[5], o, dl, dl, dl, lo, lse, status, BH, T,
-                                            scale, causal, stream);
+                                            scale, causal, cut_heads, stream);
     }
-    if (D == 64) return launch_fwd_persist<64, false>(q, nullptr, k, nullptr, v, nullptr, o, lq, lk, lv, lo, lse, status, BH, T, scale, causal, stream);
-    return launch_fwd_persist<128, false>(q, nullptr, k, nullptr, v, nullptr, o, lq, lk, lv, lo, lse, status, BH, T, scale, causal, stream);
+    if (D == 64) return launch_fwd_persist<64, false>(q, nullptr, k, nullptr, v, nullptr, o, lq, lk, lv, lo, lse, status, BH, T, scale, causal, cut_heads, stream);
+    return launch_fwd_persist<128, false>(q, nullptr, k, nullptr, v, nullptr, o, lq, lk, lv, lo, lse, status, BH, T, scale, causal, cut_heads, stream);
 }
 
 int bwd_core(const void* q, const void* k, const void* v, const void* o, const void* dO, const float* lse, void* dq, void* dk, void* dv,
@@ -769,7 +771,7 @@ int ib200_attn_fwd(const void* q, const void* k, const void* v, void* o, float* 
                    float scale, int causal, int dtype, int math_mode, void* workspace, size_t workspace_bytes,
                    ib200_stream_t stream) {
     return fwd_core(q, k, v, o, lse, nullptr, nullptr, nullptr, nullptr, B, H, T, D, scale, causal, dtype, math_mode, workspace,
-                    workspace_bytes, reinterpret_cast<cudaStream_t>(stream));
+                    workspace_bytes, 0, reinterpret_cast<cudaStream_t>(stream));
 }
 
 int ib200_attn_fwd_strided(const void* q, const void* k, const void* v, void* o, float* lse, const ib200_layout* lq,
@@ -777,7 +779,16 @@ int ib200_attn_fwd_strided(const void* q, const void* k, const void* v, void* o,
                            float scale, int causal, int dtype, int math_mode, void* workspace, size_t workspace_bytes,
                            ib200_stream_t stream) {
     return fwd_core(q, k, v, o, lse, lq, lk, lv, lo, B, H, T, D, scale, causal, dtype, math_mode, workspace, workspace_bytes,
-                    reinterpret_cast<cudaStream_t>(stream));
+                    0, reinterpret_cast<cudaStream_t>(stream));
+}
+
+int ib200_attn_fwd_chunk(const void* q, const void* k, const void* v, void* o, float* lse, const ib200_layout* lq,
+                         const ib200_layout* lk, const ib200_layout* lv, const ib200_layout* lo, int total_heads, int B, int H, int T,
+                         int D, float scale, int causal, int dtype, int math_mode, void* workspace, size_t workspace_bytes,
+                         ib200_stream_t stream) {
+    if (total_heads <= 0) return IB200_ERR_INVALID_ARGUMENT;
+    return fwd_core(q, k, v, o, lse, lq, lk, lv, lo, B, H, T, D, scale, causal, dtype, math_mode, workspace, workspace_bytes,
+                    total_heads, reinterpret_cast<cudaStream_t>(stream));
 }
 
 int ib200_attn_bwd(const void* q, const void* k, const void* v, const void* o, const void* dO, const float* lse,
@@ -785,7 +796,7 @@ int ib200_attn_bwd(const void* q, const void* k, const void* v, const void* o, c
                    int math_mode, void* workspace, size_t workspace_bytes, ib200_stream_t stream) {
     const ib200_layout* lay[8] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
     return bwd_core(q, k, v, o, dO, lse, dq, dk, dv, lay, B, H, T, D, scale, causal, dtype, math_mode, workspace, workspace_bytes,
-                    false, reinterpret_cast<cudaStream_t>(stream));
+                    0, reinterpret_cast<cudaStream_t>(stream));
 }
 
 int ib200_attn_bwd_strided(const void* q, const void* k, const void* v, const void* o, const void* dO, const float* lse,
@@ -795,7 +806,7 @@ int ib200_attn_bwd_strided(const void* q, const void* k, const void* v, const vo
                            void* workspace, size_t workspace_bytes, ib200_stream_t stream) {
     const ib200_layout* lay[8] = {lq, lk, lv, lo, ldo, ldq, ldk, ldv};
     return bwd_core(q, k, v, o, dO, lse, dq, dk, dv, lay, B, H, T, D, scale, causal, dtype, math_mode, workspace, workspace_bytes,
-                    false, reinterpret_cast<cudaStream_t>(stream));
+                    0, reinterpret_cast<cudaStream_t>(stream));
 }
 
 int ib200_attn_bwd_static(const void* q, const void* k, const void* v, const void* o, const void* dO, const float* lse,

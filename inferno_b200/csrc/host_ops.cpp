@@ -42,6 +42,7 @@ using torch::autograd::variable_list;
 struct Abi {
     decltype(&ib200_attn_workspace_bytes) workspace_bytes = nullptr;
     decltype(&ib200_attn_fwd_strided) attn_fwd = nullptr;
+    decltype(&ib200_attn_fwd_chunk) attn_fwd_chunk = nullptr;
     decltype(&ib200_attn_bwd_strided) attn_bwd = nullptr;
     decltype(&ib200_linear_workspace_bytes) linear_workspace_bytes = nullptr;
     decltype(&ib200_linear_fwd_ws) linear_fwd = nullptr;
@@ -175,7 +176,7 @@ float scale_of(const std::optional<double>& s, int64_t D) { return static_cast<f
 
 // ---- launches (the caller has made the tensors' device current) ------------------------------------------
 void launch_fwd(const Shape& s, const Operand& q, const Operand& k, const Operand& v, const Operand& o, float* lse, float scale, bool causal,
-                int math_mode, c10::Device device) {
+                int math_mode, c10::Device device, int total_heads = 0) {
     size_t bytes = 0;
     check_status(g_abi.workspace_bytes(s.B, s.H, s.T, s.D, s.dtype, IB200_PASS_FWD, &bytes), "ib200_attn_workspace_bytes");
     cudaStream_t stream = c10::cuda::getCurrentCUDAStream(device.index()).stream();
@@ -183,6 +184,12 @@ void launch_fwd(const Shape& s, const Operand& q, const Operand& k, const Operan
     std::lock_guard<std::mutex> lock(ws.launching);
     reserve(ws, bytes, device);
     TimingScope timing(false);
+    if (total_heads > 0) {
+        check_status(g_abi.attn_fwd_chunk(q.ptr, k.ptr, v.ptr, o.ptr, lse, &q.lay, &k.lay, &v.lay, &o.lay, total_heads, s.B, s.H, s.T, s.D, scale, causal,
+                                          s.dtype, math_mode, ws.buf.data_ptr(), ws.buf.numel(), reinterpret_cast<ib200_stream_t>(stream)),
+                     "ib200_attn_fwd_chunk");
+        return;
+    }
     check_status(g_abi.attn_fwd(q.ptr, k.ptr, v.ptr, o.ptr, lse, &q.lay, &k.lay, &v.lay, &o.lay, s.B, s.H, s.T, s.D, scale, causal, s.dtype, math_mode,
                                 ws.buf.data_ptr(), ws.buf.numel(), reinterpret_cast<ib200_stream_t>(stream)),
                  "ib200_attn_fwd_strided");
@@ -212,7 +219,7 @@ Tensor empty_bthd(const Tensor& q, const Shape& s) {
 
 // Forward on [B, H, T, D] tensors or views.
 std::pair<Tensor, Tensor> attention_forward(const Tensor& q_, const Tensor& k_, const Tensor& v_, const std::optional<double>& scale, bool causal,
-                                            int math_mode, const Tensor& out, const Tensor& lse_, bool bthd) {
+                                            int math_mode, const Tensor& out, const Tensor& lse_, bool bthd, int total_heads = 0) {
     check_inputs({&q_, &k_, &v_});
     const c10::cuda::CUDAGuard guard(q_.device());
     const Tensor q = dense_or_view(q_), k = dense_or_view(k_), v = dense_or_view(v_);
@@ -221,7 +228,7 @@ std::pair<Tensor, Tensor> attention_forward(const Tensor& q_, const Tensor& k_, 
     if (lse_.defined()) check_lse(lse_, q);
     Tensor o = out.defined() ? out : bthd ? empty_bthd(q, s) : at::empty(q.sizes(), q.options());
     Tensor lse = lse_.defined() ? lse_ : empty_lse(q, s);
-    launch_fwd(s, operand(q), operand(k), operand(v), operand(o), lse.data_ptr<float>(), scale_of(scale, s.D), causal, math_mode, q.device());
+    launch_fwd(s, operand(q), operand(k), operand(v), operand(o), lse.data_ptr<float>(), scale_of(scale, s.D), causal, math_mode, q.device(), total_heads);
     return {o, lse};
 }
 
@@ -556,6 +563,7 @@ PyObject* py_bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
         };
         get(g_abi.workspace_bytes, "ib200_attn_workspace_bytes");
         get(g_abi.attn_fwd, "ib200_attn_fwd_strided");
+        get(g_abi.attn_fwd_chunk, "ib200_attn_fwd_chunk");
         get(g_abi.attn_bwd, "ib200_attn_bwd_strided");
         get(g_abi.linear_workspace_bytes, "ib200_linear_workspace_bytes");
         get(g_abi.linear_fwd, "ib200_linear_fwd_ws");
@@ -569,20 +577,21 @@ PyObject* py_bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
     });
 }
 
-// (q, k, v, scale, causal, math_mode, out, lse) -> (o, lse)
+// (q, k, v, scale, causal, math_mode, out, lse, total_heads) -> (o, lse); total_heads: 0, or the heads of the problem that this call is a chunk of
 PyObject* py_attention_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     return guarded([&]() -> PyObject* {
-        want(n, 8);
+        want(n, 9);
         const Tensor &q = arg_tensor(a[0]), &k = arg_tensor(a[1]), &v = arg_tensor(a[2]);
         const auto scale = arg_scale(a[3]);
         const bool causal = arg_bool(a[4]);
         const int math_mode = static_cast<int>(arg_int(a[5]));
         const Tensor out = arg_opt_tensor(a[6]), lse = arg_opt_tensor(a[7]);
+        const int total_heads = static_cast<int>(arg_int(a[8]));
         std::pair<Tensor, Tensor> r;
         {
             pybind11::gil_scoped_release nogil;
             at::AutoDispatchBelowADInplaceOrView below;
-            r = attention_forward(q, k, v, scale, causal, math_mode, out, lse, false);
+            r = attention_forward(q, k, v, scale, causal, math_mode, out, lse, false, total_heads);
         }
         return wrap_tuple({&r.first, &r.second});
     });

@@ -7,13 +7,14 @@ Here the same round trip is chunked over heads and pipelined on three streams --
 copies, kernels, device-to-host copies -- with double-buffered device staging, so that the copies
 of one chunk overlap the kernels of another.  A staging set's input half is released as soon as the
 kernels have consumed it and its output half once the results have left, so neither copy direction
-ever waits for the other.  Heads are independent: chunking changes at most
-the rounding of O, where the forward cuts the list of a chunk differently from that of all heads.
+ever waits for the other.  Heads are independent and a chunk is walked as a
+call on all heads would be, so chunking changes nothing.
 """
 from __future__ import annotations
 
 import torch
 
+from . import _capi
 from . import attention as A
 
 
@@ -59,7 +60,7 @@ class HostAttention:
                 self.s_run.wait_event(self.ev_in[j])
                 if used[j]:
                     self.s_run.wait_event(self.ev_out[j])      # the results of that chunk have been copied out of this set
-                A.attention_forward(b["q"][:n], b["k"][:n], b["v"][:n], out=b["o"][:n], lse=b["lse"][:n])
+                _capi.host().attention_forward(b["q"][:n], b["k"][:n], b["v"][:n], None, True, _capi.MATH_SPLIT_BF16, b["o"][:n], b["lse"][:n], heads)
                 A.attention_backward(b["q"][:n], b["k"][:n], b["v"][:n], b["o"][:n], b["do"][:n], b["lse"][:n],
                                      dq=b["dq"][:n], dk=b["dk"][:n], dv=b["dv"][:n])
                 self.ev_run[j].record(self.s_run)

@@ -29,3 +29,15 @@ def test_pipeline_matches_resident_path(heads, hc, T, D):
         assert torch.equal(hout[0], o.cpu())
         assert torch.equal(hout[2], dk.cpu()) and torch.equal(hout[3], dv.cpu())
         assert float((hout[1].float() - dq.cpu().float()).abs().max()) <= 1e-2 * float(dq.float().abs().max())
+
+
+def test_chunk_of_a_large_problem_is_walked_like_the_whole():
+    """One head alone would be walked in single query tiles, 600 heads in pairs: as a chunk, one head must give the bits of the 600."""
+    from inferno_b200 import _capi
+    one = [torch.randn((1, 1, 700, 64), device="cuda").to(torch.bfloat16) for _ in range(3)]
+    o, lse = _capi.host().attention_forward(*one, None, True, _capi.MATH_SPLIT_BF16, None, None, 600)
+    o2, lse2 = A.attention_forward(*(t.expand(600, 1, 700, 64).contiguous() for t in one))
+    torch.cuda.synchronize()
+    assert torch.equal(o[0], o2[599]) and torch.equal(lse[0], lse2[599])
+    with pytest.raises(_capi.Ib200Error):
+        _capi.host().attention_forward(*(t.expand(3, 1, 700, 64).contiguous() for t in one), None, True, _capi.MATH_SPLIT_BF16, None, None, 2)
