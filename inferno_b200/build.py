@@ -56,8 +56,10 @@ def build_host(force: bool = False) -> str:
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
     for d in inc:
         cmd += ["-isystem", d]
+    # The C++ runtime has to be the shared one that torch is linked against: a compiler that comes with the static one only would
+    # put a second copy into the module, and the first error message formatted with torch's inline code then crashes the process.
     cmd += host_sources() + ["-o", HOST_PATH, "-L" + os.path.join(root, "lib"), "-ltorch_python", "-ltorch_cpu", "-ltorch_cuda",
-                             "-lc10_cuda", "-lc10", "-ldl"]
+                             "-lc10_cuda", "-lc10", "-ldl", "-nostdlib++", "-l:libstdc++.so.6"]
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError("building " + HOST_PATH + " failed:\n" + res.stdout + res.stderr)

@@ -190,3 +190,14 @@ def test_python_host_side_rejects_cpu_tensors(built_lib):
         A.attention_forward(q, q, q)
     with pytest.raises(ValueError):
         A.attention_forward(q[0], q[0], q[0])
+
+
+def test_refusals_with_formatted_messages_raise(built_lib):
+    """A message put together from numbers reaches Python as an exception (in a child process, which a mixed-up C++ runtime would kill)."""
+    import subprocess
+    import sys
+    code = ("import torch\nfrom inferno_b200 import attention as A\n"
+            "try:\n    A.causal_attention_packed(torch.zeros(1, 3, 8), 5)\n"
+            "except RuntimeError as e:\n    assert 'last axis (8)' in str(e)\nelse:\n    raise SystemExit('not refused')\n")
+    res = subprocess.run([sys.executable, "-c", code], cwd=ROOT, env=dict(os.environ, PYTHONPATH=ROOT), capture_output=True, text=True, timeout=300)
+    assert res.returncode == 0, res.stderr[-2000:]
