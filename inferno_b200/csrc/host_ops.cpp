@@ -20,6 +20,7 @@
 
 #include <dlfcn.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <deque>
@@ -388,6 +389,14 @@ Tensor causal_attention_packed(const Tensor& qkv, int64_t H, const std::optional
 }
 
 // ---- projections -------------------------------------------------------------------
+// Shapes first, ahead of any allocation: the kernels get no more than the pointers and M, K, N.
+void check_linear_shapes(const Tensor& x, const Tensor& w) {
+    TORCH_CHECK_VALUE(w.dim() == 2, "linear: w must be [in, out]");
+    TORCH_CHECK_VALUE(x.dim() >= 1 && x.size(-1) == w.size(0), "linear: the last axis of x must be w's first (", w.size(0), "), x is ", x.sizes());
+}
+void check_same_device(const Tensor& t, const Tensor& x, const char* name) {
+    TORCH_CHECK_VALUE(t.device() == x.device(), "linear: ", name, " is on ", t.device(), ", x on ", x.device());
+}
 void check_bf16_cuda(const Tensor& t, const char* name) {
     TORCH_CHECK(t.is_cuda(), "linear: ", name, " is not on a CUDA device (there is no CPU path)");
     TORCH_CHECK_TYPE(t.scalar_type() == at::kBFloat16, "linear: ", name, " must be bfloat16");
@@ -397,11 +406,14 @@ void check_bf16_cuda(const Tensor& t, const char* name) {
 constexpr size_t kHeaderBytes = 256;
 
 Tensor linear_forward(const Tensor& x, const Tensor& w, const Tensor& bias) {
+    check_linear_shapes(x, w);
+    const int64_t K = w.size(0), N = w.size(1);
+    TORCH_CHECK_VALUE(!bias.defined() || bias.numel() == N, "linear: the bias must have ", N, " elements");
     check_bf16_cuda(x, "x");
     check_bf16_cuda(w, "w");
-    TORCH_CHECK_VALUE(w.dim() == 2, "linear: w must be [in, out]");
+    check_same_device(w, x, "w");
+    if (bias.defined()) check_same_device(bias, x, "the bias");
     const c10::cuda::CUDAGuard guard(x.device());
-    const int64_t K = w.size(0), N = w.size(1);
     const Tensor x2 = x.reshape({-1, K}).contiguous(), wc = w.contiguous();
     Tensor b = bias;
     if (b.defined() && b.scalar_type() != at::kBFloat16) b = b.to(at::kFloat);
@@ -430,12 +442,16 @@ struct LinearGrads {
     Tensor dx, dw, db;
 };
 LinearGrads linear_backward(const Tensor& x, const Tensor& w, const Tensor& dy, bool need_dx, bool need_dw, bool need_db, bool db_bf16) {
+    check_linear_shapes(x, w);
+    const int64_t K = w.size(0), N = w.size(1);
+    TORCH_CHECK_VALUE(dy.dim() >= 1 && dy.size(-1) == N && dy.numel() / std::max<int64_t>(N, 1) == x.numel() / std::max<int64_t>(K, 1),
+                      "linear: dy must have the rows of x and ", N, " columns, dy is ", dy.sizes(), ", x is ", x.sizes());
     check_bf16_cuda(x, "x");
     check_bf16_cuda(w, "w");
     check_bf16_cuda(dy, "dy");
-    TORCH_CHECK_VALUE(w.dim() == 2, "linear: w must be [in, out]");
+    check_same_device(w, x, "w");
+    check_same_device(dy, x, "dy");
     const c10::cuda::CUDAGuard guard(x.device());
-    const int64_t K = w.size(0), N = w.size(1);
     const Tensor x2 = x.reshape({-1, K}).contiguous(), dy2 = dy.reshape({-1, N}).contiguous(), wc = w.contiguous();
     const int M = static_cast<int>(x2.size(0));
     LinearGrads g;
