@@ -418,6 +418,8 @@ Tensor linear_forward(const Tensor& x, const Tensor& w, const Tensor& bias) {
     Tensor b = bias;
     if (b.defined() && b.scalar_type() != at::kBFloat16) b = b.to(at::kFloat);
     if (b.defined()) b = b.contiguous();
+    // the kernel reads a bias in place: a bf16 slice that does not begin on 16 bytes is copied, as it was when every bias became fp32
+    if (b.defined() && b.scalar_type() == at::kBFloat16 && (reinterpret_cast<uintptr_t>(b.data_ptr()) & 15u)) b = b.clone();
     auto shape = x.sizes().vec();
     shape.back() = N;
     Tensor y = at::empty(shape, x.options());

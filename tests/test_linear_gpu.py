@@ -92,3 +92,12 @@ def test_tile_edges_and_split_products(M, K, N):
     assert rel(dw.double(), xd.t() @ dyd) < tol and rel(dw1.double(), xd.t() @ dyd) < tol
     assert db.dtype == torch.bfloat16 and rel(db.double(), dyd.sum(0)) < tol
     assert rel(db32.double(), dyd.sum(0)) < 1e-5
+
+
+@pytest.mark.parametrize("offset", [1, 3, 4, 8])      # 2, 6, 8 and 16 bytes past an aligned address
+def test_bias_may_be_a_slice(offset):
+    x, w = (torch.randn(*s, device="cuda").to(torch.bfloat16) for s in ((64, 64), (64, 264)))
+    buf = torch.randn(300, device="cuda").to(torch.bfloat16)
+    b = buf[offset:offset + 264]
+    y = L.linear_forward(x, w, b)
+    assert torch.equal(y, L.linear_forward(x, w, b.clone())) and rel(y, x.float() @ w.float() + b.float()) < 1e-2
