@@ -21,7 +21,7 @@ PASS_FWD, PASS_BWD = 0, 1
 EXPORTS = (
     "ib200_attn_workspace_bytes", "ib200_attn_fwd", "ib200_attn_bwd", "ib200_attn_check",
     "ib200_status_string", "ib200_last_cuda_error", "ib200_version", "ib200_attn_set_timing_events", "ib200_attn_bwd_static", "ib200_attn_fwd_strided", "ib200_attn_fwd_chunk", "ib200_attn_bwd_strided", "ib200_gemm_bf16", "ib200_linear_fwd", "ib200_linear_bwd",
-    "ib200_cast_f32_to_bf16", "ib200_cast_bf16_to_f32", "ib200_attn_item_order", "ib200_attn_check_static",
+    "ib200_cast_f32_to_bf16", "ib200_cast_bf16_to_f32", "ib200_attn_item_order", "ib200_attn_fwd_item_rows", "ib200_attn_check_static",
     "ib200_selftest_wait_expiry", "ib200_linear_workspace_bytes", "ib200_linear_fwd_ws", "ib200_linear_bwd_ws",
 )
 
@@ -79,6 +79,8 @@ def lib() -> ctypes.CDLL:
         ip = ctypes.POINTER(ctypes.c_int)
         L.ib200_attn_item_order.argtypes = [i, i, i, i, i, i, ip, ip, i, ip]
         L.ib200_attn_item_order.restype = i
+        L.ib200_attn_fwd_item_rows.argtypes = [i, i, i, i]
+        L.ib200_attn_fwd_item_rows.restype = i
         L.ib200_attn_check.argtypes = [vp, vp, ctypes.POINTER(i)]
         L.ib200_attn_check.restype = i
         L.ib200_attn_check_static.argtypes = [vp, ctypes.POINTER(i)]

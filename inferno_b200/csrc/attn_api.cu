@@ -680,13 +680,19 @@ extern "C" {
 
 int ib200_version(void) { return 1001; }
 
+int ib200_attn_fwd_item_rows(int total_heads, int T, int causal, int sm_count) {
+    if (total_heads <= 0 || T <= 0 || sm_count <= 0 || (causal != 0 && causal != 1)) return -IB200_ERR_INVALID_ARGUMENT;
+    return fwd_one_tile(total_heads, T, causal, sm_count) ? 128 : 256;
+}
+
 int ib200_attn_item_order(int pass, int B, int H, int T, int D, int sm_count, int* heads, int* units, int capacity, int* n_groups) {
     if (B <= 0 || H <= 0 || T <= 0 || sm_count <= 0 || capacity < 0 || (capacity > 0 && (!heads || !units))) return -IB200_ERR_INVALID_ARGUMENT;
     if (D != 64 && D != 128) return -IB200_ERR_UNSUPPORTED;
     if (pass != IB200_PASS_FWD && pass != IB200_PASS_BWD) return -IB200_ERR_INVALID_ARGUMENT;
     const long BH = static_cast<long>(B) * H;
     const bool fwd = pass == IB200_PASS_FWD;
-    const int per_head = fwd ? (T + 255) / 256 : (T + 127) / 128;       // query-tile pairs / key tiles
+    const int rows = fwd && !fwd_one_tile(BH, T, 1, sm_count) ? 256 : 128;
+    const int per_head = (T + rows - 1) / rows;                         // pairs of query tiles or query tiles / key tiles
     const long items = per_head * BH;
     if (BH > 65535 || items > 0x7fffffffL) return -IB200_ERR_UNSUPPORTED;
     const int groups = persist_head_groups(sm_count, per_head, BH, static_cast<size_t>(T) * D * (fwd ? 4 : 8));
@@ -696,7 +702,7 @@ int ib200_attn_item_order(int pass, int B, int H, int T, int D, int sm_count, in
         int rank, bh;
         locate_item(hg, static_cast<int>(i), rank, bh);
         heads[i] = bh;
-        units[i] = fwd ? per_head - 1 - rank : rank;                      // the longest walk first: last pair / first key tile
+        units[i] = fwd ? per_head - 1 - rank : rank;                      // the longest walk first: last pair or query tile / first key tile
     }
     return static_cast<int>(items);
 }

@@ -293,14 +293,17 @@ def _eval64(q, k, v, causal):
 
 
 # One head leaves SMs idle: its query tiles are separate items and two softmax groups share a tile's keys.  148 x 4 copies of it
-# are walked in pairs of tiles.  One to ten key tiles (odd and even, past the ring of two or four), a last tile of one row, exact tiles.
-@pytest.mark.parametrize("T", [128, 129, 255, 257, 384, 513, 640, 1161])
+# are walked in pairs of tiles.  Two to eleven key tiles (odd and even, past the ring of two or four), a last tile of one row, exact
+# tiles; one key tile at most is always walked as a pair whose second tile is empty.
+@pytest.mark.parametrize("T", [1300, 129, 255, 257, 384, 513, 640, 1161])
 @pytest.mark.parametrize("dt,D", [("bf16", 64), ("bf16", 128), ("f32", 64)])
 @pytest.mark.parametrize("causal", [True, False])
 def test_single_tile_items_and_tile_pairs_agree(T, dt, D, causal):
     q, k, v = (torch.from_numpy(a).cuda().to(TDT[dt]) for a in make_inputs(1, 1, T, D, 300 + T, 1.5, 1.0, dt)[:3])
     ref, lse_ref = _eval64(q, k, v, causal)
     many = [t.expand(148, 4, T, D).contiguous() for t in (q, k, v)]
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert [_capi.lib().ib200_attn_fwd_item_rows(n, T, int(causal), sms) for n in (1, 148 * 4)] == [128, 256]
     runs = [A.attention_forward(q, k, v, causal=causal), A.attention_forward(*many, causal=causal)]
     torch.cuda.synchronize()
     A.check_device_status()

@@ -172,6 +172,22 @@ def test_item_order_of_persistent_kernels(built_lib, case):
     assert L.ib200_attn_item_order(7, B, H, T, D, sms, heads, units, n, None) == -_capi.ERR_INVALID_ARGUMENT
 
 
+# Forwards that leave SMs idle, or whose longest walk is longer than an SM's average load, are walked in single query tiles.
+@pytest.mark.parametrize("B,H,T,D", [(1, 12, 200, 64), (1, 4, 4096, 128), (1, 12, 4096, 128), (3, 5, 777, 128), (1, 1, 129, 64)])
+def test_item_order_lists_single_tiles_where_the_forward_walks_them(built_lib, B, H, T, D):
+    L = _capi.lib()
+    assert L.ib200_attn_fwd_item_rows(B * H, T, 1, 148) == 128
+    per_head = (T + 127) // 128
+    n = B * H * per_head
+    heads, units, groups = (ctypes.c_int * n)(), (ctypes.c_int * n)(), ctypes.c_int(0)
+    assert L.ib200_attn_item_order(0, B, H, T, D, 148, heads, units, n, ctypes.byref(groups)) == n
+    assert sorted(zip(heads, units)) == [(h, u) for h in range(B * H) for u in range(per_head)]
+    assert groups.value == 1 and list(units) == sorted(units, reverse=True)          # longest walk first
+    # the same heads as a part of many are walked in pairs
+    assert L.ib200_attn_fwd_item_rows(16384, T, 1, 148) == 256
+    assert L.ib200_attn_fwd_item_rows(0, T, 1, 148) == L.ib200_attn_fwd_item_rows(1, T, 2, 148) == -_capi.ERR_INVALID_ARGUMENT
+
+
 def test_no_device_fails_loudly(built_lib):
     """With well-formed arguments and no sm_100 device the call reports it; nothing else runs."""
     import torch
