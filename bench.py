@@ -13,7 +13,8 @@ at every N), copy them in, W warm-up steps, further untimed steps until the GPU 
 --min-load-seconds (so that every N is timed in the same, settled power state), EXACTLY K timed steps between two
 CUDA events, the end-to-end pipeline and its copy-only floor, and -- outside every timed region -- the validation:
 each rank checks the first and last head of its shard against a float64 evaluation, 64-bit checksums of O, dK and dV
-of every head are gathered over NCCL, and their digest is printed (it must not depend on N).
+of every head are gathered over NCCL, and their digest is printed (it must not depend on N: every rank passes the
+number of heads of the whole problem to the forward, which is what its order of summation depends on).
 For N > 1 launch with torchrun (one rank per GPU); a bare `python bench.py --gpus N` re-launches itself.
 """
 from __future__ import annotations
@@ -409,7 +410,7 @@ def run_ours(args, cfg):
     flush_buf = torch.empty(256 << 20, dtype=torch.uint8, device=dev) if flush else None
 
     def step():
-        A.attention_forward(q, k, v, out=o, lse=lse)
+        A.attention_forward(q, k, v, out=o, lse=lse, total_heads=BH)
         A.attention_backward(q, k, v, o, do, lse, dq=dq, dk=dk, dv=dv)
 
     def barrier():
@@ -507,7 +508,7 @@ def run_ours(args, cfg):
     if args.e2e_steps <= 0:      # profiling runs only; a bench line without e2e is not a result
         e2e = None
     else:
-        e2e = measure_e2e(args, torch, dist, HostAttention, dev, world, n, T, D, tdt, host_in, (o, dk, dv), barrier, total_flops)
+        e2e = measure_e2e(args, torch, dist, HostAttention, dev, world, BH, n, T, D, tdt, host_in, (o, dk, dv), barrier, total_flops)
 
     if rank != 0:
         if world > 1:
@@ -516,18 +517,18 @@ def run_ours(args, cfg):
     finish(args, cfg, world, n, T, D, K, W, preload_steps, value, ms_step, fwd_ms_max, bwd_ms_max, clocks, e2e, validation, graph, dist)
 
 
-def measure_e2e(args, torch, dist, HostAttention, dev, world, n, T, D, tdt, hin, resident, barrier, total_flops):
+def measure_e2e(args, torch, dist, HostAttention, dev, world, BH, n, T, D, tdt, hin, resident, barrier, total_flops):
     hc = args.e2e_heads_per_chunk if args.e2e_heads_per_chunk > 0 else max(1, n // 8)
     hc = max(1, min(n, hc))
     pipe = HostAttention(hc, T, D, tdt, dev, nbuf=args.e2e_nbuf)
     hout = [torch.empty((n, 1, T, D), dtype=tdt).pin_memory() for _ in range(4)]
-    pipe.run(*hin, *hout)                      # warm-up (also first touch of the pinned pages)
+    pipe.run(*hin, *hout, total_heads=BH)             # warm-up (also first touch of the pinned pages)
     barrier()
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     Ke = max(1, args.e2e_steps)
     e0.record()
     for _ in range(Ke):
-        pipe.run(*hin, *hout, wait=False)
+        pipe.run(*hin, *hout, wait=False, total_heads=BH)
     e1.record()
     barrier()
     # the floor: the same copies over the same buffers and chunks, both directions at once, no kernels, all ranks at once
@@ -539,7 +540,7 @@ def measure_e2e(args, torch, dist, HostAttention, dev, world, n, T, D, tdt, hin,
         pipe.copy_only(*hin, *hout)
     c1.record()
     barrier()
-    pipe.run(*hin, *hout)                      # leave real results in the host buffers for the check below
+    pipe.run(*hin, *hout, total_heads=BH)             # leave real results in the host buffers for the check below
     te = torch.tensor([e0.elapsed_time(e1) / Ke, c0.elapsed_time(c1) / Ke], device=dev, dtype=torch.float64)
     if world > 1:
         dist.all_reduce(te, op=dist.ReduceOp.MAX)

@@ -42,12 +42,16 @@ def _raise(rc: int, where: str):
 
 
 def attention_forward(q, k, v, scale: float | None = None, causal: bool = True, math_mode: int = _capi.MATH_SPLIT_BF16,
-                      out=None, lse=None):
+                      out=None, lse=None, total_heads: int | None = None):
     """Launch the forward kernel.  Returns (o [B,H,T,D], lse [B,H,T] fp32).  Asynchronous on the current stream.
+
+    ``total_heads``: the heads of the whole problem when this call computes a part of them (a shard, a chunk).  The order in which
+    a row's keys are summed depends on how many heads there are; given the whole number, a head gets the bits that one call on
+    all heads would give it.
 
     q, k, v (and ``out``) may be arbitrary [B,H,T,D] views with a contiguous last axis -- e.g. slices of a packed
     [B,T,3,H,D] projection, or an output laid out [B,T,H,D] -- and are then read and written in place."""
-    return _capi.host().attention_forward(q, k, v, scale, causal, math_mode, out, lse, 0)
+    return _capi.host().attention_forward(q, k, v, scale, causal, math_mode, out, lse, total_heads)
 
 
 def attention_backward(q, k, v, o, dO, lse, scale: float | None = None, causal: bool = True,
@@ -109,19 +113,21 @@ class AttentionBackward:
 
     @staticmethod
     def apply(q, k, v, scale, causal, math_mode, bthd_out):
-        return _capi.host().causal_attention(q, k, v, scale, causal, math_mode, bthd_out)
+        return _capi.host().causal_attention(q, k, v, scale, causal, math_mode, bthd_out, None)
 
 
 def causal_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, scale: float | None = None,
-                     math_mode: int = _capi.MATH_SPLIT_BF16, bthd_out: bool = False) -> torch.Tensor:
-    """``softmax(mask(q k^T * scale)) v`` with a causal mask; differentiable.  q, k, v: [B,H,T,D] tensors or views."""
-    return _capi.host().causal_attention(q, k, v, scale, True, math_mode, bthd_out)
+                     math_mode: int = _capi.MATH_SPLIT_BF16, bthd_out: bool = False, total_heads: int | None = None) -> torch.Tensor:
+    """``softmax(mask(q k^T * scale)) v`` with a causal mask; differentiable.  q, k, v: [B,H,T,D] tensors or views.
+    ``total_heads`` as in ``attention_forward``."""
+    return _capi.host().causal_attention(q, k, v, scale, True, math_mode, bthd_out, total_heads)
 
 
 def causal_attention_packed(qkv: torch.Tensor, num_heads: int, scale: float | None = None,
-                            math_mode: int = _capi.MATH_SPLIT_BF16) -> torch.Tensor:
+                            math_mode: int = _capi.MATH_SPLIT_BF16, total_heads: int | None = None) -> torch.Tensor:
     """Attention straight on the fused projection output: ``qkv`` is [B, T, 3*C] (= [B,T,3,H,D]); returns [B, T, C].
     Replaces slice / contiguous / reshape / transpose / contiguous before the kernels and transpose / contiguous /
     reshape after them (InfernoApp/main.cpp:716-737, 758-761) with stride arithmetic: no copy kernel runs, and the
-    gradient is written into one [B, T, 3*C] buffer by the kernels themselves."""
-    return _capi.host().causal_attention_packed(qkv, num_heads, scale, math_mode)
+    gradient is written into one [B, T, 3*C] buffer by the kernels themselves.  ``total_heads`` (batch times heads of the
+    whole problem) as in ``attention_forward``."""
+    return _capi.host().causal_attention_packed(qkv, num_heads, scale, math_mode, total_heads)

@@ -293,13 +293,14 @@ struct AttentionBackward : torch::autograd::Node {
     std::string name() const override { return "AttentionBackward"; }
 };
 
-Tensor causal_attention(const Tensor& q, const Tensor& k, const Tensor& v, const std::optional<double>& scale, bool causal, int math_mode, bool bthd) {
+Tensor causal_attention(const Tensor& q, const Tensor& k, const Tensor& v, const std::optional<double>& scale, bool causal, int math_mode, bool bthd,
+                        int total_heads) {
     refuse_tangents({&q, &k, &v}, "causal_attention");
     const bool differentiable = torch::autograd::compute_requires_grad(q, k, v);
     Tensor o, lse;
     {
         at::AutoDispatchBelowADInplaceOrView below;
-        std::tie(o, lse) = attention_forward(q, k, v, scale, causal, math_mode, Tensor(), Tensor(), bthd);
+        std::tie(o, lse) = attention_forward(q, k, v, scale, causal, math_mode, Tensor(), Tensor(), bthd, total_heads);
     }
     if (differentiable) {
         auto node = std::shared_ptr<AttentionBackward>(new AttentionBackward(), torch::autograd::deleteNode);
@@ -351,7 +352,7 @@ struct PackedAttentionBackward : torch::autograd::Node {
     std::string name() const override { return "PackedAttentionBackward"; }
 };
 
-Tensor causal_attention_packed(const Tensor& qkv, int64_t H, const std::optional<double>& scale, int math_mode) {
+Tensor causal_attention_packed(const Tensor& qkv, int64_t H, const std::optional<double>& scale, int math_mode, int total_heads) {
     TORCH_CHECK_VALUE(qkv.dim() == 3 && H > 0, "causal_attention_packed expects a [B, T, 3*C] tensor and a positive number of heads");
     const int64_t B = qkv.size(0), T = qkv.size(1), C = qkv.size(2) / 3, D = C / H;
     TORCH_CHECK(3 * D * H == qkv.size(2), "causal_attention_packed: the last axis (", qkv.size(2), ") is not 3 * num_heads * head_dim");
@@ -372,7 +373,7 @@ Tensor causal_attention_packed(const Tensor& qkv, int64_t H, const std::optional
         o = at::empty({B, T, C}, p.options());
         lse = at::empty({B, H, T}, p.options().dtype(at::kFloat));
         launch_fwd(s, packed_operand(p, 0, C, D), packed_operand(p, 1, C, D), packed_operand(p, 2, C, D), packed_operand(o, 0, C, D), lse.data_ptr<float>(),
-                   scale_of(scale, D), true, math_mode, p.device());
+                   scale_of(scale, D), true, math_mode, p.device(), total_heads);
     }
     if (differentiable) {
         auto node = std::shared_ptr<PackedAttentionBackward>(new PackedAttentionBackward(), torch::autograd::deleteNode);
@@ -532,6 +533,13 @@ int64_t arg_int(PyObject* o) {
     if (v == -1 && PyErr_Occurred()) throw python_error();
     return v;
 }
+// None (0): the call is the whole problem; otherwise the heads of the problem that it is a part of.
+int arg_total_heads(PyObject* o) {
+    if (o == Py_None) return 0;
+    const int64_t n = arg_int(o);
+    TORCH_CHECK_VALUE(n > 0 && n <= 0x7fffffff, "causal_attention: total_heads must be a positive number of heads, got ", n);
+    return static_cast<int>(n);
+}
 bool arg_bool(PyObject* o) {
     const int v = PyObject_IsTrue(o);
     if (v < 0) throw python_error();
@@ -595,7 +603,7 @@ PyObject* py_bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
     });
 }
 
-// (q, k, v, scale, causal, math_mode, out, lse, total_heads) -> (o, lse); total_heads: 0, or the heads of the problem that this call is a chunk of
+// (q, k, v, scale, causal, math_mode, out, lse, total_heads) -> (o, lse)
 PyObject* py_attention_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     return guarded([&]() -> PyObject* {
         want(n, 9);
@@ -604,7 +612,7 @@ PyObject* py_attention_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const bool causal = arg_bool(a[4]);
         const int math_mode = static_cast<int>(arg_int(a[5]));
         const Tensor out = arg_opt_tensor(a[6]), lse = arg_opt_tensor(a[7]);
-        const int total_heads = static_cast<int>(arg_int(a[8]));
+        const int total_heads = arg_total_heads(a[8]);
         std::pair<Tensor, Tensor> r;
         {
             pybind11::gil_scoped_release nogil;
@@ -634,36 +642,38 @@ PyObject* py_attention_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     });
 }
 
-// (q, k, v, scale, causal, math_mode, bthd_out) -> y, differentiable
+// (q, k, v, scale, causal, math_mode, bthd_out, total_heads) -> y, differentiable
 PyObject* py_causal_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
     return guarded([&]() -> PyObject* {
-        want(n, 7);
+        want(n, 8);
         const Tensor &q = arg_tensor(a[0]), &k = arg_tensor(a[1]), &v = arg_tensor(a[2]);
         const auto scale = arg_scale(a[3]);
         const bool causal = arg_bool(a[4]);
         const int math_mode = static_cast<int>(arg_int(a[5]));
         const bool bthd = arg_bool(a[6]);
+        const int total_heads = arg_total_heads(a[7]);
         Tensor y;
         {
             pybind11::gil_scoped_release nogil;
-            y = causal_attention(q, k, v, scale, causal, math_mode, bthd);
+            y = causal_attention(q, k, v, scale, causal, math_mode, bthd, total_heads);
         }
         return wrap(y);
     });
 }
 
-// (qkv, num_heads, scale, math_mode) -> y, differentiable
+// (qkv, num_heads, scale, math_mode, total_heads) -> y, differentiable
 PyObject* py_causal_attention_packed(PyObject*, PyObject* const* a, Py_ssize_t n) {
     return guarded([&]() -> PyObject* {
-        want(n, 4);
+        want(n, 5);
         const Tensor& qkv = arg_tensor(a[0]);
         const int64_t H = arg_int(a[1]);
         const auto scale = arg_scale(a[2]);
         const int math_mode = static_cast<int>(arg_int(a[3]));
+        const int total_heads = arg_total_heads(a[4]);
         Tensor y;
         {
             pybind11::gil_scoped_release nogil;
-            y = causal_attention_packed(qkv, H, scale, math_mode);
+            y = causal_attention_packed(qkv, H, scale, math_mode, total_heads);
         }
         return wrap(y);
     });

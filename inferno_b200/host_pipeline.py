@@ -7,14 +7,13 @@ Here the same round trip is chunked over heads and pipelined on three streams --
 copies, kernels, device-to-host copies -- with double-buffered device staging, so that the copies
 of one chunk overlap the kernels of another.  A staging set's input half is released as soon as the
 kernels have consumed it and its output half once the results have left, so neither copy direction
-ever waits for the other.  Heads are independent and a chunk is walked as a
-call on all heads would be, so chunking changes nothing.
+ever waits for the other.  Heads are independent and a chunk is walked as a call on all heads would
+be, so chunking changes nothing.
 """
 from __future__ import annotations
 
 import torch
 
-from . import _capi
 from . import attention as A
 
 
@@ -36,12 +35,14 @@ class HostAttention:
         self.ev_out = [torch.cuda.Event() for _ in range(nbuf)]
         self.ev_done = torch.cuda.Event()
 
-    def run(self, q, k, v, do, o, dq, dk, dv, wait: bool = True) -> None:
+    def run(self, q, k, v, do, o, dq, dk, dv, wait: bool = True, total_heads: int | None = None) -> None:
         """All arguments: pinned host tensors [heads, 1, T, D] (or any shape with that many elements per head).
         With ``wait`` (the default) the call returns after every output has landed in host memory; with
         ``wait=False`` the results are only ordered on the caller's current stream, and the host must synchronise
-        that stream (or call ``wait_done``) before it reads the output tensors."""
+        that stream (or call ``wait_done``) before it reads the output tensors.  ``total_heads``: the heads of the whole
+        problem when these are a shard of them (``attention_forward``)."""
         heads = q.shape[0]
+        whole = heads if total_heads is None else total_heads
         main = torch.cuda.current_stream(self.device)
         for s in (self.s_in, self.s_run, self.s_out):
             s.wait_stream(main)
@@ -60,7 +61,7 @@ class HostAttention:
                 self.s_run.wait_event(self.ev_in[j])
                 if used[j]:
                     self.s_run.wait_event(self.ev_out[j])      # the results of that chunk have been copied out of this set
-                _capi.host().attention_forward(b["q"][:n], b["k"][:n], b["v"][:n], None, True, _capi.MATH_SPLIT_BF16, b["o"][:n], b["lse"][:n], heads)
+                A.attention_forward(b["q"][:n], b["k"][:n], b["v"][:n], out=b["o"][:n], lse=b["lse"][:n], total_heads=whole)
                 A.attention_backward(b["q"][:n], b["k"][:n], b["v"][:n], b["o"][:n], b["do"][:n], b["lse"][:n],
                                      dq=b["dq"][:n], dk=b["dk"][:n], dv=b["dv"][:n])
                 self.ev_run[j].record(self.s_run)

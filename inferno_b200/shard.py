@@ -3,7 +3,9 @@
 Attention is independent per (batch, head): outputs and gradients of one head depend only on
 that head's Q, K, V and dO.  Multi-GPU runs therefore give each rank a contiguous range of the
 B*H heads -- a contiguous slab of every dense [B,H,T,D] tensor -- and need no collective inside
-the attention path.  (The reference is single-process and single-GPU; it has no counterpart.)
+the attention path.  The order in which the forward sums a row depends on the number of heads of the
+problem, so a rank passes the whole number (``total_heads`` of the attention entry points): its heads
+then get the bits that one GPU would give them.  (The reference is single-process and single-GPU; it has no counterpart.)
 """
 from __future__ import annotations
 

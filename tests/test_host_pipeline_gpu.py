@@ -41,3 +41,42 @@ def test_chunk_of_a_large_problem_is_walked_like_the_whole():
     assert torch.equal(o[0], o2[599]) and torch.equal(lse[0], lse2[599])
     with pytest.raises(_capi.Ib200Error):
         _capi.host().attention_forward(*(t.expand(3, 1, 700, 64).contiguous() for t in one), None, True, _capi.MATH_SPLIT_BF16, None, None, 2)
+
+
+# Configurations whose shards, cut by their own number of heads, would be walked in single query tiles where the whole is walked in pairs.
+@pytest.mark.parametrize("B,H,T,D,dt,ranks", [(2, 16, 8192, 128, torch.bfloat16, 8), (8, 12, 1024, 64, torch.float32, 8), (16, 12, 1024, 64, torch.bfloat16, 8)])
+def test_shards_get_the_bits_of_the_whole(B, H, T, D, dt, ranks):
+    from inferno_b200 import _capi
+    from inferno_b200.shard import shard_range
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    rows = [_capi.lib().ib200_attn_fwd_item_rows(n, T, 1, sms) for n in (B * H, B * H // ranks)]
+    assert rows == [256, 128]
+    g = torch.Generator(device="cuda").manual_seed(3)
+    q, k, v, do = (torch.randn(B * H, 1, T, D, device="cuda", generator=g).to(dt) for _ in range(4))
+    o, lse = A.attention_forward(q, k, v)
+    _, dk, dv = A.attention_backward(q, k, v, o, do, lse)
+    for r in range(ranks):
+        s = slice(shard_range(B * H, r, ranks).start, shard_range(B * H, r, ranks).stop)
+        o1, lse1 = A.attention_forward(q[s], k[s], v[s], total_heads=B * H)
+        _, dk1, dv1 = A.attention_backward(q[s], k[s], v[s], o1, do[s], lse1)
+        assert all(torch.equal(a, b[s]) for a, b in ((o1, o), (lse1, lse), (dk1, dk), (dv1, dv)))
+    assert torch.equal(A.causal_attention(q[s], k[s], v[s], total_heads=B * H), o[s])
+
+
+def test_packed_op_and_host_pipeline_take_the_number_of_heads_of_the_whole():
+    B, H, T, D, heads = 1, 4, 700, 64, 600
+    g = torch.Generator(device="cuda").manual_seed(4)
+    qkv = torch.randn(B, T, 3 * H * D, device="cuda", generator=g).to(torch.bfloat16)
+    many = A.causal_attention_packed(qkv.expand(150, T, 3 * H * D).contiguous(), H)
+    assert torch.equal(A.causal_attention_packed(qkv, H, total_heads=heads)[0], many[149])
+    q, k, v = (qkv.view(B, T, 3, H, D)[:, :, i].transpose(1, 2).reshape(B * H, 1, T, D) for i in range(3))
+    hin = [t.cpu().pin_memory() for t in (q, k, v, q)]
+    hout = [torch.empty_like(hin[0]).pin_memory() for _ in range(4)]
+    HostAttention(2, T, D, torch.bfloat16, "cuda").run(*hin, *hout, total_heads=heads)
+    assert torch.equal(hout[0].view(H, T, D).transpose(0, 1).reshape(T, H * D), many[149].cpu())
+    for bad in (0, -1, 2 ** 40):
+        with pytest.raises(ValueError, match="total_heads"):
+            A.causal_attention_packed(qkv, H, total_heads=bad)
+    for call in (lambda: A.causal_attention_packed(qkv, H, total_heads=3), lambda: A.attention_forward(q, k, v, total_heads=3)):
+        with pytest.raises(Exception, match="invalid argument"):      # fewer heads than the call itself has
+            call()
