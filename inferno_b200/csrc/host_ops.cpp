@@ -139,10 +139,19 @@ void check_like(const Tensor& t, const Tensor& q, const char* name) {
                       "` must match q in shape, dtype and device");
 }
 // The log-sum-exp vector is addressed densely by the kernels.
-void check_lse(const Tensor& lse, const Tensor& q) {
-    TORCH_CHECK_VALUE(lse.scalar_type() == at::kFloat && lse.device() == q.device() && lse.dim() == 3 && lse.size(0) == q.size(0) &&
-                          lse.size(1) == q.size(1) && lse.size(2) == q.size(2) && lse.is_contiguous(),
+void check_lse_of(const Tensor& lse, c10::Device device, int64_t B, int64_t H, int64_t T) {
+    TORCH_CHECK_VALUE(lse.scalar_type() == at::kFloat && lse.device() == device && lse.dim() == 3 && lse.size(0) == B && lse.size(1) == H &&
+                          lse.size(2) == T && lse.is_contiguous(),
                       "causal_attention: `lse` must be a contiguous float32 [B, H, T] tensor on q's device");
+}
+void check_lse(const Tensor& lse, const Tensor& q) { check_lse_of(lse, q.device(), q.size(0), q.size(1), q.size(2)); }
+// A packed [B, T, 3*H*D] operand.
+void check_packed(const Tensor& qkv, int64_t H) {
+    TORCH_CHECK_VALUE(qkv.dim() == 3 && H > 0, "causal_attention_packed expects a [B, T, 3*C] tensor and a positive number of heads");
+    TORCH_CHECK(qkv.size(2) / 3 / H * H * 3 == qkv.size(2), "causal_attention_packed: the last axis (", qkv.size(2), ") is not 3 * num_heads * head_dim");
+    TORCH_CHECK(qkv.is_cuda(), "causal_attention: tensor is not on a CUDA device (there is no CPU path)");
+    TORCH_CHECK_TYPE(qkv.scalar_type() == at::kFloat || qkv.scalar_type() == at::kBFloat16,
+                     "causal_attention: dtype must be float32 or bfloat16, the same for all tensors");
 }
 
 // A [B, H, T, D] operand as the C ABI takes it.
@@ -160,6 +169,13 @@ Tensor dense_or_view(const Tensor& t) {
     const int64_t unit = 16 / t.element_size();
     bool ok = t.stride(3) == 1 && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15u) == 0;
     for (int a = 0; a < 3; ++a) ok = ok && t.stride(a) > 0 && t.stride(a) % unit == 0;
+    return ok ? t : t.contiguous();
+}
+// The same for a packed [B, T, n*H*D] tensor.
+Tensor dense_or_packed(const Tensor& t) {
+    const int64_t unit = 16 / t.element_size();
+    const bool ok = t.stride(2) == 1 && t.stride(0) > 0 && t.stride(1) > 0 && t.stride(0) % unit == 0 && t.stride(1) % unit == 0 &&
+                    (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15u) == 0;
     return ok ? t : t.contiguous();
 }
 // One third of a packed [B, T, 3, H, D] buffer, as a [B, H, T, D] operand.
@@ -329,17 +345,20 @@ struct PackedAttentionBackward : torch::autograd::Node {
 
     variable_list apply(variable_list&& grads) override {
         if (!grads[0].defined()) return variable_list(1);
-        const Tensor p = qkv.unpack(), to = o.unpack(shared_from_this()), tl = lse.unpack();
+        const Tensor p_ = qkv.unpack(), o_ = o.unpack(shared_from_this()), tl = lse.unpack();
         at::AutoDispatchBelowADInplaceOrView below;
-        const c10::cuda::CUDAGuard guard(p.device());
-        const int64_t B = p.size(0), T = p.size(1), C = p.size(2) / 3, D = C / H;
+        // what was saved has passed through the user's saved-tensor hooks, and may come back with other strides, or as something else
+        check_packed(p_, H);
+        const c10::cuda::CUDAGuard guard(p_.device());
+        const int64_t B = p_.size(0), T = p_.size(1), C = p_.size(2) / 3, D = C / H;
+        for (const Tensor& t : {o_, grads[0]}) {
+            TORCH_CHECK(t.device() == p_.device(), "causal_attention: tensors are on different devices");
+            TORCH_CHECK_TYPE(t.scalar_type() == p_.scalar_type(), "causal_attention: dtype must be float32 or bfloat16, the same for all tensors");
+            TORCH_CHECK_VALUE(t.dim() == 3 && t.size(0) == B && t.size(1) == T && t.size(2) == C, "causal_attention: the output and its gradient must be [B, T, C]");
+        }
+        check_lse_of(tl, p_.device(), B, H, T);
+        const Tensor p = dense_or_packed(p_), to = dense_or_packed(o_), dy = dense_or_packed(grads[0]);
         const Shape s{static_cast<int>(B), static_cast<int>(H), static_cast<int>(T), static_cast<int>(D), dtype_code(p)};
-        Tensor dy = grads[0];
-        const int64_t unit = 16 / dy.element_size();
-        TORCH_CHECK_TYPE(dy.scalar_type() == p.scalar_type(), "causal_attention: dtype must be float32 or bfloat16, the same for all tensors");
-        if (dy.stride(2) != 1 || dy.stride(0) <= 0 || dy.stride(1) <= 0 || dy.stride(0) % unit || dy.stride(1) % unit ||
-            (reinterpret_cast<uintptr_t>(dy.data_ptr()) & 15u))
-            dy = dy.contiguous();
         Tensor g = at::empty({B, T, 3 * C}, p.options());
         launch_bwd(s, packed_operand(p, 0, C, D), packed_operand(p, 1, C, D), packed_operand(p, 2, C, D), packed_operand(to, 0, C, D),
                    packed_operand(dy, 0, C, D), tl.data_ptr<float>(), packed_operand(g, 0, C, D), packed_operand(g, 1, C, D), packed_operand(g, 2, C, D), scale,
@@ -353,22 +372,15 @@ struct PackedAttentionBackward : torch::autograd::Node {
 };
 
 Tensor causal_attention_packed(const Tensor& qkv, int64_t H, const std::optional<double>& scale, int math_mode, int total_heads) {
-    TORCH_CHECK_VALUE(qkv.dim() == 3 && H > 0, "causal_attention_packed expects a [B, T, 3*C] tensor and a positive number of heads");
+    check_packed(qkv, H);
     const int64_t B = qkv.size(0), T = qkv.size(1), C = qkv.size(2) / 3, D = C / H;
-    TORCH_CHECK(3 * D * H == qkv.size(2), "causal_attention_packed: the last axis (", qkv.size(2), ") is not 3 * num_heads * head_dim");
-    TORCH_CHECK(qkv.is_cuda(), "causal_attention: tensor is not on a CUDA device (there is no CPU path)");
-    TORCH_CHECK_TYPE(qkv.scalar_type() == at::kFloat || qkv.scalar_type() == at::kBFloat16,
-                     "causal_attention: dtype must be float32 or bfloat16, the same for all tensors");
     refuse_tangents({&qkv}, "causal_attention");
     const bool differentiable = torch::autograd::compute_requires_grad(qkv);
     Tensor o, lse, p;
     {
         at::AutoDispatchBelowADInplaceOrView below;
         const c10::cuda::CUDAGuard guard(qkv.device());
-        const int64_t unit = 16 / qkv.element_size();
-        const bool ok = qkv.stride(2) == 1 && qkv.stride(0) > 0 && qkv.stride(1) > 0 && qkv.stride(0) % unit == 0 && qkv.stride(1) % unit == 0 &&
-                        (reinterpret_cast<uintptr_t>(qkv.data_ptr()) & 15u) == 0;
-        p = ok ? qkv : qkv.contiguous();
+        p = dense_or_packed(qkv);
         const Shape s{static_cast<int>(B), static_cast<int>(H), static_cast<int>(T), static_cast<int>(D), dtype_code(p)};
         o = at::empty({B, T, C}, p.options());
         lse = at::empty({B, H, T}, p.options().dtype(at::kFloat));

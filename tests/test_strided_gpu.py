@@ -118,3 +118,29 @@ def test_ops_refuse_tangents_and_save_through_hooks():
     torch.autograd.grad((y.float().sum() + z.float().sum()), (x, qkv))
     torch.cuda.synchronize()
     A.check_device_status()
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float32])
+def test_saved_tensor_hooks_may_change_the_layout_and_nothing_else(dt):
+    """What a hook hands back is checked like any operand: other strides are copied, another place, type or shape is refused."""
+    B, T, H, D = 2, 150, 2, 64
+    g = torch.Generator(device="cuda").manual_seed(8)
+    qkv = torch.randn(B, T, 3 * H * D, device="cuda", generator=g).to(dt).requires_grad_()
+    dy = torch.randn(B, T, H * D, device="cuda", generator=g).to(dt)
+    want, = torch.autograd.grad(A.causal_attention_packed(qkv, H), qkv, dy)
+
+    def through(pack, unpack=lambda t: t):
+        with torch.autograd.graph.saved_tensors_hooks(pack, unpack):
+            y = A.causal_attention_packed(qkv, H)
+        return torch.autograd.grad(y, qkv, dy)[0]
+
+    other_strides = lambda t: t if t.shape == (B, H, T) else t.transpose(0, 2).contiguous().transpose(0, 2)       # lse is [B, H, T]
+    got = through(other_strides)
+    assert torch.equal(got[..., H * D:], want[..., H * D:])                     # dK, dV; dQ is summed in varying order
+    assert (got - want).float().norm() <= 1e-3 * want.float().norm()
+    wider = lambda t: t.double()
+    for pack in (lambda t: t.cpu(), wider, lambda t: t[:1], lambda t: t.transpose(0, 1), lambda t: t.flatten()):
+        with pytest.raises((RuntimeError, TypeError, ValueError)):
+            through(pack)
+    torch.cuda.synchronize()
+    A.check_device_status()
