@@ -54,8 +54,8 @@ struct Abi {
 };
 Abi g_abi;
 
-// A status other than IB200_OK from the library.  On the caller's thread it becomes the package's own exception type; out of
-// a backward node (autograd's worker thread) it surfaces as the RuntimeError that type derives from.
+// A status other than IB200_OK from the library.  It reaches Python as the package's own exception type, from the caller's thread
+// (guarded) and from autograd's worker threads (in_node) alike.
 struct StatusError : std::runtime_error {
     int status;
     const char* where;
@@ -271,6 +271,27 @@ Grads attention_backward(const Tensor& q_, const Tensor& k_, const Tensor& v_, c
 }
 
 // ---- autograd nodes ----------------------------------------------------------------
+void set_python_error(const StatusError& e) {      // with the GIL
+    PyObject* err = PyObject_CallFunction(g_abi.error_class, "is", e.status, e.where);
+    if (!err) return;
+    PyErr_SetObject(g_abi.error_class, err);
+    Py_DECREF(err);
+}
+// Body of a node: a status becomes a Python exception that the engine carries over to the thread that called backward.
+template <class F>
+variable_list in_node(F&& f) {
+    try {
+        return f();
+    } catch (const StatusError& e) {
+        python_error err;
+        {
+            pybind11::gil_scoped_acquire gil;
+            set_python_error(e);
+            err.persist();
+        }
+        throw err;
+    }
+}
 // The ops have no forward-mode derivative: a dual input must not lose its tangent silently.
 void refuse_tangents(std::initializer_list<const Tensor*> ts, const char* op) {
     for (const Tensor* t : ts)
@@ -286,6 +307,9 @@ struct AttentionBackward : torch::autograd::Node {
     int math_mode = 0;
 
     variable_list apply(variable_list&& grads) override {
+        return in_node([&] { return backward(grads); });
+    }
+    variable_list backward(const variable_list& grads) {
         if (!grads[0].defined()) return variable_list(3);
         const Tensor tq = q.unpack(), tk = k.unpack(), tv = v.unpack(), to = o.unpack(shared_from_this()), tl = lse.unpack();
         at::AutoDispatchBelowADInplaceOrView below;
@@ -344,6 +368,9 @@ struct PackedAttentionBackward : torch::autograd::Node {
     int math_mode = 0;
 
     variable_list apply(variable_list&& grads) override {
+        return in_node([&] { return backward(grads); });
+    }
+    variable_list backward(const variable_list& grads) {
         if (!grads[0].defined()) return variable_list(1);
         const Tensor p_ = qkv.unpack(), o_ = o.unpack(shared_from_this()), tl = lse.unpack();
         at::AutoDispatchBelowADInplaceOrView below;
@@ -492,6 +519,9 @@ struct LinearBackward : torch::autograd::Node {
     at::ScalarType bias_type = at::kFloat;
 
     variable_list apply(variable_list&& grads) override {
+        return in_node([&] { return backward(grads); });
+    }
+    variable_list backward(const variable_list& grads) {
         variable_list out(3);
         if (!grads[0].defined()) return out;
         const Tensor tx = x.unpack(), tw = w.unpack();
@@ -578,11 +608,7 @@ PyObject* guarded(F&& f) {
     try {
         return f();
     } catch (const StatusError& e) {
-        PyObject* err = PyObject_CallFunction(g_abi.error_class, "is", e.status, e.where);
-        if (err) {
-            PyErr_SetObject(g_abi.error_class, err);
-            Py_DECREF(err);
-        }
+        set_python_error(e);
         return nullptr;
     }
     END_HANDLE_TH_ERRORS

@@ -144,3 +144,20 @@ def test_saved_tensor_hooks_may_change_the_layout_and_nothing_else(dt):
             through(pack)
     torch.cuda.synchronize()
     A.check_device_status()
+
+
+def test_a_status_in_a_backward_node_is_the_packages_own_error():
+    """A library status reaches the caller of backward as Ib200Error with its number, as it does from a forward call."""
+    from inferno_b200 import _capi
+    from inferno_b200.linear import Linear
+    bf16 = lambda *s: torch.randn(*s, device="cuda").to(torch.bfloat16).requires_grad_()
+    # what is saved comes back two bytes off an aligned address, which the library refuses
+    off = lambda t: t if t.dtype == torch.float32 else torch.cat([t.flatten()[:1], t.flatten()])[1:].view(t.shape)
+    q, qkv, x, lin = bf16(1, 2, 64, 64), bf16(1, 64, 384), bf16(64, 128), Linear(128, 64).cuda().to(torch.bfloat16)
+    for leaf, call in ((q, lambda: A.causal_attention(q, q, q)), (qkv, lambda: A.causal_attention_packed(qkv, 2)), (x, lambda: lin(x))):
+        with torch.autograd.graph.saved_tensors_hooks(off, lambda t: t):
+            y = call()
+        with pytest.raises(_capi.Ib200Error) as e:
+            torch.autograd.grad(y.float().sum(), leaf)
+        assert e.value.status == _capi.ERR_MISALIGNED
+    torch.cuda.synchronize()
