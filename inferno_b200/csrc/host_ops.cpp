@@ -29,6 +29,8 @@
 #include <mutex>
 #include <optional>
 #include <string>
+#include <utility>
+#include <vector>
 
 #include "../../include/inferno_b200_attn.h"
 
@@ -764,14 +766,22 @@ PyObject* py_linear_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
 // () -> {(device index, stream handle): workspace tensor}
 PyObject* py_workspaces(PyObject*, PyObject* const*, Py_ssize_t) {
     return guarded([&]() -> PyObject* {
+        std::vector<std::pair<std::pair<int, int64_t>, Tensor>> list;
+        {
+            // A launch holds its entry's lock without the GIL and may come to need it there (to free a buffer that Python has seen, or
+            // to allocate under a Python dispatch mode), so nobody waits for that lock with the GIL in hand.
+            pybind11::gil_scoped_release nogil;
+            std::lock_guard<std::mutex> lock(g_ws_mutex);
+            for (const auto& [key, ws] : workspace_table()) {
+                std::lock_guard<std::mutex> launching(ws->launching);
+                if (ws->buf.defined()) list.emplace_back(key, ws->buf);
+            }
+        }
         PyObject* out = PyDict_New();
         if (!out) throw python_error();
-        std::lock_guard<std::mutex> lock(g_ws_mutex);
-        for (const auto& [key, ws] : workspace_table()) {
-            std::lock_guard<std::mutex> launching(ws->launching);
-            if (!ws->buf.defined()) continue;
+        for (const auto& [key, buf] : list) {
             PyObject* k = Py_BuildValue("(iL)", key.first, static_cast<long long>(key.second));
-            PyObject* v = wrap(ws->buf);
+            PyObject* v = wrap(buf);
             if (k && v) PyDict_SetItem(out, k, v);
             Py_XDECREF(k);
             Py_XDECREF(v);
@@ -784,10 +794,9 @@ PyObject* py_workspaces(PyObject*, PyObject* const*, Py_ssize_t) {
 PyObject* py_queue_timing_events(PyObject*, PyObject* const* a, Py_ssize_t n) {
     return guarded([&]() -> PyObject* {
         want(n, 2);
-        std::lock_guard<std::mutex> lock(g_timing.m);
+        std::deque<std::pair<cudaEvent_t, cudaEvent_t>> queues[2];      // filled first: reading a sequence may run Python code, which must not happen under the lock
         for (int i = 0; i < 2; ++i) {
-            auto& q = i ? g_timing.bwd : g_timing.fwd;
-            q.clear();
+            auto& q = queues[i];
             PyObject* seq = PySequence_Fast(a[i], "expected a sequence of event pairs");
             if (!seq) throw python_error();
             for (Py_ssize_t j = 0; j < PySequence_Fast_GET_SIZE(seq); ++j) {
@@ -800,6 +809,9 @@ PyObject* py_queue_timing_events(PyObject*, PyObject* const* a, Py_ssize_t n) {
             }
             Py_DECREF(seq);
         }
+        std::lock_guard<std::mutex> lock(g_timing.m);
+        g_timing.fwd.swap(queues[0]);
+        g_timing.bwd.swap(queues[1]);
         g_timing.any = !g_timing.fwd.empty() || !g_timing.bwd.empty();
         Py_RETURN_NONE;
     });

@@ -119,3 +119,31 @@ def test_range_checked_build_runs_the_small_shapes_clean(oracle_mod):
     res = subprocess.run([sys.executable, "-c", _BOUNDS_SCRIPT], env=env, cwd=ROOT, capture_output=True, text=True, timeout=600)
     assert res.returncode == 0, res.stdout[-2000:] + res.stderr[-4000:]
     assert "all cases clean" in res.stdout
+
+
+_STATUS_THREAD_SCRIPT = r"""
+import threading, torch
+from inferno_b200 import attention as A
+done = threading.Event()
+def look():
+    while not done.is_set():
+        A._workspace._bufs
+watcher = threading.Thread(target=look)
+watcher.start()
+with torch.cuda.stream(torch.cuda.Stream()):
+    for T in range(64, 64 * 60, 64):            # every call needs a larger workspace than the one before
+        x = torch.randn(1, 2, T, 64, device="cuda")
+        A.attention_forward(x, x, x)
+done.set()
+watcher.join()
+torch.cuda.synchronize()
+A.check_device_status()
+print("both threads came to an end")
+"""
+
+
+def test_reading_the_status_does_not_stop_a_thread_that_grows_its_workspace():
+    """A thread that looks at the workspaces (which hands them to Python) beside one that replaces them; in a child process, with a time limit."""
+    res = subprocess.run([sys.executable, "-c", _STATUS_THREAD_SCRIPT], env=dict(os.environ, PYTHONPATH=ROOT), cwd=ROOT, capture_output=True,
+                         text=True, timeout=120)
+    assert res.returncode == 0 and "came to an end" in res.stdout, res.stdout[-500:] + res.stderr[-2000:]
