@@ -183,11 +183,11 @@ int persist_head_groups(int ctas, int items_per_head, long BH, size_t shared_byt
 
 // Persistent CTAs walking (head, query-tile pair) items, or with ONE_TILE (head, query tile) items, heaviest first.  SPLIT: fp32 I/O, operands given as dense
 // (hi, lo) bf16 copies (q_lo, k_lo, v_lo), output fp32.
-template <int D, bool SPLIT, bool ONE_TILE>
+template <int D, bool SPLIT, bool ONE_TILE, bool CLAIM_EARLY>
 int launch_fwd_items(const void* q, const void* q_lo, const void* k, const void* k_lo, const void* v, const void* v_lo, void* o,
                        const RowLayout& lq, const RowLayout& lk, const RowLayout& lv, const RowLayout& lo, float* lse, int* status,
                        long BH, int T, float scale, int causal, cudaStream_t stream) {
-    using TR = FwdPersistTraits<D, SPLIT, ONE_TILE>;
+    using TR = FwdPersistTraits<D, SPLIT, ONE_TILE, CLAIM_EARLY>;
     CUtensorMap tq, tql, tk, tkl, tv, tvl, to;
     if (!make_tmap(&tq, q, false, D, T, lq, BH, 128) || !make_tmap(&tk, k, false, D, T, lk, BH, 128) ||
         !make_tmap(&tv, v, false, D, T, lv, BH, 128) || !make_tmap(&to, o, SPLIT, D, T, lo, BH, 128))
@@ -244,13 +244,23 @@ bool fwd_one_tile(long BH, int T, int causal, int sms) {
     return ones < pairs;
 }
 
+// When a CTA asks for its next item: late (with the last loads of the current one) the end of a short list comes out even, early
+// (with the first) a long one runs quicker.  It is not the claim's latency (a late request 2, 4 or 8 key tiles sooner changed nothing); what
+// else separates the two was not found.  Forward, us, late / early, bf16 at full clock:
+//   rounds of items   7: 473 / 493 (D = 128, T = 8192), 118 / 115 (T = 1024)   14: 912 / 922, 501 / 501 (T = 4096), 764 / 754 (D = 64)
+//                    21: 736 / 729   28: 967 / 958, 1756 / 1752 (T = 8192), 370 / 364 (T = 1024)   55: 1903 / 1879   111: 3767 / 3697, D = 64 3124 / 3085
+// At the power cap the last line's D = 128 is 4361 / 4266.  fp32 operands: late at every length (28 rounds: 1525 / 1546).
+bool fwd_claims_early(long items, int sms) { return items >= 16L * sms; }
+
 template <int D, bool SPLIT>
 int launch_fwd_persist(const void* q, const void* q_lo, const void* k, const void* k_lo, const void* v, const void* v_lo, void* o,
                        const RowLayout& lq, const RowLayout& lk, const RowLayout& lv, const RowLayout& lo, float* lse, int* status,
                        long BH, int T, float scale, int causal, long cut_heads, cudaStream_t stream) {
     const DeviceInfo* dev = device_info();
     if (!dev) return IB200_ERR_CUDA;
-    auto launch = fwd_one_tile(cut_heads, T, causal, dev->sms) ? launch_fwd_items<D, SPLIT, true> : launch_fwd_items<D, SPLIT, false>;
+    auto launch = fwd_one_tile(cut_heads, T, causal, dev->sms) ? launch_fwd_items<D, SPLIT, true, false> : launch_fwd_items<D, SPLIT, false, false>;
+    if constexpr (!SPLIT)
+        if (launch == launch_fwd_items<D, SPLIT, false, false> && fwd_claims_early(BH * ((T + 255) / 256), dev->sms)) launch = launch_fwd_items<D, SPLIT, false, true>;
     return launch(q, q_lo, k, k_lo, v, v_lo, o, lq, lk, lv, lo, lse, status, BH, T, scale, causal, stream);
 }
 

@@ -26,10 +26,12 @@ namespace ib200 {
 
 // ONE_TILE: an item is one query tile, and the two softmax groups take its key tiles in turn (group 0 the even ones, group 1
 // the odd ones), each with its own S, O, maximum and sum; the epilogue puts the two halves together.
-template <int D_, bool SPLIT_ = false, bool ONE_TILE_ = false>
+// CLAIM_EARLY: the next item is asked for with an item's first loads instead of its last (the host decides: fwd_claims_early).  A
+// kernel of its own: with a run-time flag in the one kernel the long list that gains 1.6 % by it lost 1 %.
+template <int D_, bool SPLIT_ = false, bool ONE_TILE_ = false, bool CLAIM_EARLY_ = false>
 struct FwdPersistTraits : FwdTraits<D_, SPLIT_> {
     using Base = FwdTraits<D_, SPLIT_>;
-    static constexpr bool ONE_TILE = ONE_TILE_;
+    static constexpr bool ONE_TILE = ONE_TILE_, CLAIM_EARLY = CLAIM_EARLY_;
     static constexpr int BM_ITEM = ONE_TILE ? 128 : 256;
     // ONE_TILE: each group writes one 128-byte panel of the output; where there is only one, group 0 writes it
     static constexpr bool BOTH_WRITE = ONE_TILE && Base::OUT_PANELS == 2;
@@ -165,11 +167,16 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                     for (int p = 0; p < TR::NP; ++p)
                         tma_load_4d(sK + ((G + j) % KS) * TR::TILE_BYTES + p * TR::PANEL_BYTES, (TR::SPLIT && p) ? &tm_k_lo : &tm_k, q_full, col(p), j * BN, it.hd,
                                     it.bt);
+                if constexpr (TR::CLAIM_EARLY) {
+                    item_request(source);
+                    idx = item_take(source, n, pp.n_items, ab);
+                    item_ring_publish(ring, n, idx, ab);
+                }
                 for (int j = 0; j < it.n_iter; ++j, ++G) {
                     const int s = G % KS;
                     const bool has_k = (j + kAhead) < it.n_iter;
                     mbar_wait(&kv_empty[s], ((G / KS) & 1) ^ 1, ab, 10);
-                    if (j + 1 == it.n_iter) item_request(source);        // KS key tiles before the item's end (see ItemSource)
+                    if (!TR::CLAIM_EARLY && j + 1 == it.n_iter) item_request(source);        // KS key tiles before the item's end (see ItemSource)
                     // K_KS reuses the slot of K_0 (ONE_TILE: and K_KS+1 that of K_1, which k0_free covers too)
                     if (j == KS - kAhead && (kAhead == 1 || has_k)) mbar_wait(k0_free, n & 1, ab, 11);
                     mbar_arrive_expect_tx(&kv_full[s], (has_k ? 2 : 1) * TR::TILE_BYTES);
@@ -180,8 +187,10 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                     for (int p = 0; p < TR::NP; ++p)
                         tma_load_4d(sV + s * TR::TILE_BYTES + p * TR::PANEL_BYTES, (TR::SPLIT && p) ? &tm_v_lo : &tm_v, &kv_full[s], col(p), j * BN, it.hd, it.bt);
                 }
-                idx = item_take(source, n, pp.n_items, ab);
-                item_ring_publish(ring, n, idx, ab);
+                if constexpr (!TR::CLAIM_EARLY) {
+                    idx = item_take(source, n, pp.n_items, ab);
+                    item_ring_publish(ring, n, idx, ab);
+                }
             }
             pdl_trigger();      // this CTA's last loads are out: the next kernel may start as the SMs empty (triggered at the start instead, the next
                                 // kernel's waiting CTAs cost the backward 5-10 %)

@@ -344,3 +344,20 @@ def test_single_tile_items_keep_infinities():
         assert torch.equal(torch.isnan(x), torch.isnan(ref[0, 0])) and torch.equal(torch.isnan(l), torch.isnan(lse_ref[0, 0]))
         ok = ~torch.isnan(lse_ref[0, 0])
         assert (x[ok].double() - ref[0, 0][ok]).norm() / ref[0, 0][ok].norm() < 2 * 2.0 ** -8
+
+
+@pytest.mark.parametrize("T,D", [(200, 64), (256, 128), (300, 128)])
+def test_lists_either_side_of_the_early_claim_agree(T, D):
+    """A list of 16 rounds of items or more is walked by the kernel that claims early: the same bits as one item fewer."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    units = (T + 255) // 256
+    n = 16 * sms // units
+    assert _capi.lib().ib200_attn_fwd_item_rows(n - 1, T, 1, sms) == 256
+    one = [torch.from_numpy(a).cuda().to(torch.bfloat16) for a in make_inputs(1, 1, T, D, 77, 1.0, 1.0, "bf16")[:3]]
+    ref, _ = _eval64(*one, True)
+    runs = [A.attention_forward(*(t.expand(h, 1, T, D).contiguous() for t in one)) for h in (n, n - 1)]
+    torch.cuda.synchronize()
+    A.check_device_status()
+    for o, lse in runs:
+        assert torch.equal(o, runs[0][0][:1].expand_as(o)) and torch.equal(lse, runs[0][1][:1].expand_as(lse))
+    assert (runs[0][0][0, 0].double() - ref[0, 0]).norm() / ref.norm() < 2 * 2.0 ** -8
