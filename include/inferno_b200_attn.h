@@ -187,11 +187,12 @@ int ib200_attn_check(const void* workspace, ib200_stream_t stream, int* device_c
  * check_cuda() convention (src/inferno/cuda/cudaops.h:198-210). */
 int ib200_attn_check_static(ib200_stream_t stream, int* device_code);
 
-/* Self-test of the bounded-wait machinery, for test suites: launches one small CTA that allocates
- * tensor memory and waits on a barrier nothing ever signals; after `limit_us` microseconds
- * (1 .. 100000) the wait gives up, the CTA records site code 190 in the header of `workspace`
- * (at least 256 bytes), releases its tensor memory and exits normally -- no fault, no trap; the
- * context stays usable.  ib200_attn_check on the workspace then returns
+/* Self-test of the bounded-wait machinery, for test suites: launches small CTAs, eight per SM of which one is
+ * resident at a time, that allocate tensor memory and wait on a barrier nothing ever signals; after
+ * `limit_us` microseconds (1 .. 100000) the wait gives up, the CTA records site code 190 in the
+ * header of `workspace` (at least 256 bytes), releases its tensor memory and exits normally -- no
+ * fault, no trap; the context stays usable.  CTAs that start after the report do not wait, so the
+ * launch ends after about one limit.  ib200_attn_check on the workspace then returns
  * IB200_ERR_DEVICE_TIMEOUT with *device_code == 190.  The reference has no counterpart (its
  * kernels never wait on each other). */
 int ib200_selftest_wait_expiry(void* workspace, size_t workspace_bytes, unsigned limit_us, ib200_stream_t stream);

@@ -166,6 +166,14 @@ bool allow_smem(int bytes) {
     return true;
 }
 
+// Numbers the launches of a process, so that the CTAs of one know a failure of their own (launch_failed).  Never 0.
+int next_launch_number() {
+    static std::atomic<unsigned> last{0};
+    unsigned n = last.fetch_add(1, std::memory_order_relaxed) + 1;
+    while (n == 0) n = last.fetch_add(1, std::memory_order_relaxed) + 1;
+    return static_cast<int>(n);
+}
+
 // Number of head groups of a persistent kernel's item list (see locate_item).  The CTAs draw items in list order, so at
 // any time they work on a window of about one round (one item per CTA) of the list.  With every head in one group the window
 // would span up to one head per CTA, and the tiles the CTAs of a head share (K / V in the forward; Q / dO and the dQ
@@ -204,6 +212,7 @@ int launch_fwd_items(const void* q, const void* q_lo, const void* k, const void*
     FwdPersistParams pp;
     pp.p.lse = lse;
     pp.p.status = status;
+    pp.p.launch = next_launch_number();
     pp.p.T = T;
     pp.p.BH = static_cast<int>(BH);
     pp.p.H = lq.H;
@@ -299,6 +308,7 @@ int launch_bwd_persist(const void* const q[2], const void* const k[2], const voi
     prm.ndelta = ndelta;
     prm.T_pad = T_pad;
     prm.status = status;
+    prm.launch = next_launch_number();
     prm.T = T;
     prm.BH = static_cast<int>(BH);
     prm.H = lq.H;
@@ -418,20 +428,24 @@ int static_scratch(void** out) {
 
 // Self-test of the bounded-wait path, without any fault: one CTA allocates TMEM, warp 1 waits on an mbarrier that
 // nothing ever arrives on and gives up after `limit_ns`, warp 2 waits on the same barrier with the product limit and
-// must come back as soon as warp 1 has raised the CTA's abort flag; the CTA then frees its TMEM and exits normally.
-__global__ void __launch_bounds__(128, 1) wait_expiry_probe_kernel(int* status, unsigned long long limit_ns) {
+// must come back as soon as warp 1 has raised the CTA's abort flag; the CTA then frees its TMEM and exits normally.  CTAs that start
+// after that (its shared memory lets one be resident per SM) must not wait at all.
+constexpr int kProbeSmem = 120 * 1024;
+__global__ void __launch_bounds__(128, 1) wait_expiry_probe_kernel(int* status, int launch, unsigned long long limit_ns) {
     __shared__ uint64_t bar;
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
     const int warp = threadIdx.x >> 5;
-    if (threadIdx.x == 0) { abort_flag = 0; mbar_init(&bar, 1); fence_mbar_init(); }
+    if (threadIdx.x == 0) { abort_flag = launch_failed(status, launch); mbar_init(&bar, 1); fence_mbar_init(); }
     if (warp == 0) { tmem_alloc(&tmem_slot, 32); tmem_relinquish(); }
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
-    AbortCtx ab{&abort_flag, status};
-    if (warp == 1) mbar_wait_limit(&bar, 0, ab, 90, limit_ns);
-    if (warp == 2) mbar_wait(&bar, 0, ab, 91);
+    AbortCtx ab{&abort_flag, status, launch};
+    const bool wait = abort_flag == 0;
+    __syncthreads();                     // everybody has looked before anybody raises the flag
+    if (warp == 1 && wait) mbar_wait_limit(&bar, 0, ab, 90, limit_ns);
+    if (warp == 2 && wait) mbar_wait(&bar, 0, ab, 91);
     tc_fence_before_sync();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tmem_slot, 32);
@@ -892,10 +906,11 @@ int ib200_selftest_wait_expiry(void* workspace, size_t workspace_bytes, unsigned
     cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
     if (!workspace || !aligned16(workspace) || workspace_bytes < kHeaderBytes) return IB200_ERR_WORKSPACE;
     if (limit_us == 0 || limit_us > 100000u) return IB200_ERR_INVALID_ARGUMENT;
-    int rc = device_ok();
-    if (rc != IB200_OK) return rc;
+    const DeviceInfo* dev = device_info();
+    if (!dev) return IB200_ERR_NO_DEVICE;
+    if (!allow_smem<wait_expiry_probe_kernel>(kProbeSmem)) return IB200_ERR_CUDA;
     IB200_SET_BOUNDS(0, 0, 0, 0, 0, 1, 32, static_cast<int*>(workspace), stream);
-    wait_expiry_probe_kernel<<<1, 128, 0, stream>>>(static_cast<int*>(workspace), 1000ull * limit_us);
+    wait_expiry_probe_kernel<<<8 * dev->sms, 128, kProbeSmem, stream>>>(static_cast<int*>(workspace), next_launch_number(), 1000ull * limit_us);
     return launch_status();
 }
 

@@ -94,7 +94,8 @@ struct BwdParams {
     const float* nlse2;    // [BH, T_pad]  -lse * log2(e), 0 in the padding
     const float* ndelta;   // [BH, T_pad]  -rowsum(dO * O), 0 in the padding
     int T_pad;             // T rounded up to a multiple of 64
-    int* status;
+    int* status;           // workspace header (word 0: device status, 0 = ok)
+    int launch;            // number of this launch (launch_failed)
     int T, BH, H, causal;  // H: heads per batch entry (operand tensor maps are 4-D: column, token, head, batch)
     float scale, scale_log2;
     float dq_scale;        // factor applied to every dQ^T partial before it is added: 1 when an fp32 accumulator is finished by

@@ -75,7 +75,7 @@ attn_bwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     const int BH = prm.BH;
     const int nqb = (T + BQ - 1) / BQ;
     const int n_kt = (T + BKV - 1) / BKV;
-    AbortCtx ab{abort_flag, prm.status};
+    AbortCtx ab{abort_flag, prm.status, prm.launch};
 
     // item -> head, key tile, first query block, number of query blocks (identical in every role)
     struct Item { int bh, hd, bt, n, m0, nblk; };
@@ -90,7 +90,7 @@ attn_bwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     };
 
     if (tid == 0) {
-        *abort_flag = 0;
+        const bool failed = launch_failed(prm.status, prm.launch);      // the load's latency passes under the lines below
         mbar_init(kv_full, 1);
         for (int s = 0; s < NS; ++s) { mbar_init(&qdo_full[s], 1); mbar_init(&qdo_empty[s], 1); }
         for (int b = 0; b < NB; ++b) {
@@ -101,6 +101,7 @@ attn_bwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
         mbar_init(dkv_free, 4);
         mbar_init(clc_bar, 1);
         item_ring_init(items, 13);               // readers: the MMA warp, eight compute warps, four drain warps
+        *abort_flag = failed;                    // every role then leaves its loop at once
         fence_mbar_init();
     }
     if (warp == 13) { tmem_alloc(tmem_slot, TR::TM_COLS); tmem_relinquish(); }

@@ -62,7 +62,8 @@ struct FwdTraits {
 
 struct FwdParams {
     float* lse;            // [BH, T] natural-log units, scale included
-    int* status;           // device status word (0 = ok)
+    int* status;           // workspace header (word 0: device status, 0 = ok)
+    int launch;            // number of this launch (launch_failed)
     int T, BH, H;          // H: heads per batch entry (the tensor maps are 4-D: column, token, head, batch)
     int causal;
     float scale_log2;      // scale * log2(e)

@@ -87,7 +87,7 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     const int BH = prm.BH;
     const int n_kv_total = (T + BN - 1) / BN;
     constexpr int kAhead = TR::ONE_TILE ? 2 : 1;            // load group j brings V_j and K_{j + kAhead}
-    AbortCtx ab{abort_flag, prm.status};
+    AbortCtx ab{abort_flag, prm.status, prm.launch};
 
     // item -> head, query tiles, key-tile counts (identical in every role)
     // nkv: key tiles of each softmax group; n_iter: key tiles loaded
@@ -116,7 +116,7 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     };
 
     if (tid == 0) {
-        *abort_flag = 0;
+        const bool failed = launch_failed(prm.status, prm.launch);      // the load's latency passes under the lines below
         mbar_init(q_full, 1);
         mbar_init(q_free, 1);
         mbar_init(k0_free, 1);
@@ -129,6 +129,7 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
         mbar_init(stage_free, 1);
         mbar_init(clc_bar, 1);
         item_ring_init(ring, 9);                 // readers: the MMA warp and the eight softmax warps
+        *abort_flag = failed;                    // every role then leaves its loop at once
         fence_mbar_init();
     }
     if (warp == 8) { tmem_alloc(tmem_slot, TR::TM_COLS); tmem_relinquish(); }

@@ -17,7 +17,9 @@ namespace ib200 {
 // thread for a system-dependent while, so a poll count alone does not bound time),
 // the waiter raises the CTA-wide abort flag and records a code in the kernel's global
 // status word; every later wait in that CTA returns at once, the CTA runs to its
-// normal tear-down (TMEM freed) and the host reports an error.
+// normal tear-down (TMEM freed) and the host reports an error.  A launch of more CTAs than
+// are resident at a time still ends after about one limit: a CTA that starts after a
+// report of its own launch does nothing (launch_failed).
 // ----------------------------------------------------------------------------
 constexpr uint32_t kSpinLimit = 1u << 24;
 #ifdef IB200_BOUNDS
@@ -36,14 +38,30 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
-// Header of a workspace: word 0 = device status (sticky until the host has read it), word 3 = a mark that says word 0 is a status.
-// A workspace arrives uninitialised and no launch prepares it: whoever has something to report sets the mark, and a first
-// report replaces whatever word 0 held.
+// Header of a workspace: word 0 = device status (sticky until the host has read it), word 2 = number of the last launch a CTA of
+// which gave up, word 3 = a mark that says word 0 is a status.  A workspace arrives uninitialised and no launch prepares it: whoever
+// has something to report sets the mark, and a first report replaces whatever word 0 held.
 constexpr int kHeaderMagic = 0x1b200a77;
 __device__ __forceinline__ void report_status(int* header, int code) {
     if (!header) return;
     if (atomicExch(header + 3, kHeaderMagic) != kHeaderMagic) atomicExch(header, code);
     else atomicCAS(header, 0, code);
+}
+
+// A wait that expired.  A call, not inlined: some forty waits a kernel carry it, and without the atomics in each the code is so much
+// shorter that the kernels run quicker (us: backward of 192 heads T = 1024 D = 64 173.4 -> 168.9, of 96 fp32 heads 169.5 -> 166.1 with
+// its pre-pass; forward of 16 heads T = 4096 D = 128 62.8 -> 61.7, of 1024 3701 -> 3670).
+__device__ __noinline__ void report_expiry(int* header, int launch, int code) {
+    if (!header) return;
+    if (launch != 0) atomicExch(header + 2, launch);
+    report_status(header, code);
+}
+// Has a CTA of this launch given up already?  Asked once, by a CTA that starts; the failures of other launches, read or not, do not
+// count (a CUDA graph replays its launches under their numbers: it does nothing until the host has read the status).
+__device__ __forceinline__ bool launch_failed(const int* header, int launch) {
+    int4 h;
+    asm volatile("ld.volatile.global.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(h.x), "=r"(h.y), "=r"(h.z), "=r"(h.w) : "l"(header) : "memory");
+    return h.x != 0 && h.z == launch && h.w == kHeaderMagic;
 }
 
 enum : int {
@@ -95,7 +113,8 @@ __device__ __forceinline__ bool tmem_addr_ok(uint32_t taddr, uint32_t ncols) {
 
 struct AbortCtx {
     volatile int* cta_flag;   // shared memory, one per CTA
-    int* status;              // global memory, one per launch (may be null)
+    int* status;              // global memory: header of the launch's workspace (may be null)
+    int launch;               // number of the launch, for its CTAs that start later (0: all of them are resident)
 };
 
 
@@ -168,7 +187,7 @@ __device__ __forceinline__ bool mbar_wait_limit(uint64_t* bar, uint32_t parity, 
             if (t_start == 0) t_start = now;
             if (spins > kSpinLimit || now - t_start > limit_ns) {
                 *ab.cta_flag = 1;
-                report_status(ab.status, kDevTimeoutBase + site);
+                report_expiry(ab.status, ab.launch, kDevTimeoutBase + site);
                 return false;
             }
         }

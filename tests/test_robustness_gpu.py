@@ -147,3 +147,69 @@ def test_reading_the_status_does_not_stop_a_thread_that_grows_its_workspace():
     res = subprocess.run([sys.executable, "-c", _STATUS_THREAD_SCRIPT], env=dict(os.environ, PYTHONPATH=ROOT), cwd=ROOT, capture_output=True,
                          text=True, timeout=120)
     assert res.returncode == 0 and "came to an end" in res.stdout, res.stdout[-500:] + res.stderr[-2000:]
+
+
+def test_a_launch_of_many_rounds_ends_after_one_limit():
+    """Eight rounds of CTAs that would each wait 50 ms: those that start after the first report do not wait."""
+    L = _capi.lib()
+    ws = torch.zeros(256, device="cuda", dtype=torch.uint8)
+    s = torch.cuda.current_stream().cuda_stream
+    for _ in range(2):                                  # an unread report of an earlier launch changes nothing
+        t0, t1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        t0.record()
+        assert L.ib200_selftest_wait_expiry(ws.data_ptr(), ws.numel(), 50000, s) == _capi.OK
+        t1.record()
+        torch.cuda.synchronize()
+        assert 45.0 < t0.elapsed_time(t1) < 150.0
+    assert _check(ws) == (_capi.ERR_DEVICE_TIMEOUT, 190)
+
+
+_FAILED_LAUNCH_SCRIPT = r"""
+import ctypes, torch
+from inferno_b200 import _capi
+L = _capi.lib()
+B, H, T, D = 2, 3, 300, 64
+q, k, v = (torch.randn(B, H, T, D, device="cuda").to(torch.bfloat16) for _ in range(3))
+o, want = (torch.full_like(q, 7.0) for _ in range(2))
+lse = torch.full((B, H, T), 7.0, device="cuda")
+ws = torch.zeros(_capi.workspace_bytes(B, H, T, D, _capi.DTYPE_BF16, _capi.PASS_BWD), device="cuda", dtype=torch.uint8)
+s = torch.cuda.current_stream().cuda_stream
+def fwd(out, l):
+    return L.ib200_attn_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), l.data_ptr(), B, H, T, D, 0.125, 1, _capi.DTYPE_BF16, 0,
+                            ws.data_ptr(), ws.numel(), s)
+def bwd(outs):
+    return L.ib200_attn_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), v.data_ptr(), lse.data_ptr(), *(t.data_ptr() for t in outs), B, H, T, D,
+                            0.125, 1, _capi.DTYPE_BF16, 0, ws.data_ptr(), ws.numel(), s)
+header = ws[:16].view(torch.int32)
+def report(launch):           # what a CTA of that launch leaves behind when a wait of its runs out
+    header.copy_(torch.tensor([121, 0, launch, 0x1b200a77], dtype=torch.int32))
+report(1)                     # the process' first launch
+assert fwd(o, lse) == _capi.OK
+torch.cuda.synchronize()
+assert bool((o == 7.0).all()) and bool((lse == 7.0).all())          # every CTA left at once
+assert fwd(o, lse) == _capi.OK and fwd(want, torch.empty_like(lse)) == _capi.OK          # launches 2 and 3 run, although nobody has read the report
+ref = torch.nn.functional.scaled_dot_product_attention(q.float(), k.float(), v.float(), is_causal=True)
+assert torch.equal(o, want) and float((o.float() - ref).norm() / ref.norm()) < 2e-2
+grads = [torch.full_like(q, 7.0) for _ in range(3)]
+report(4)
+assert bwd(grads) == _capi.OK
+torch.cuda.synchronize()
+assert bool((grads[1] == 7.0).all()) and bool((grads[2] == 7.0).all())
+assert bwd(grads) == _capi.OK
+torch.cuda.synchronize()
+qr, kr, vr = (t.float().requires_grad_() for t in (q, k, v))
+ref = torch.autograd.grad(torch.nn.functional.scaled_dot_product_attention(qr, kr, vr, is_causal=True), (qr, kr, vr), v.float())
+for got, want in zip(grads, ref):
+    assert float((got.float() - want).norm() / want.norm()) < 2e-2
+code = ctypes.c_int(-1)
+assert L.ib200_attn_check(ws.data_ptr(), s, ctypes.byref(code)) == _capi.ERR_DEVICE_TIMEOUT and code.value == 121
+assert L.ib200_attn_check(ws.data_ptr(), s, ctypes.byref(code)) == _capi.OK
+print("failed launches left at once")
+"""
+
+
+def test_ctas_of_a_failed_launch_leave_at_once():
+    """A forward and a backward whose header already holds a report of their own launch touch nothing; the launches after them run."""
+    res = subprocess.run([sys.executable, "-c", _FAILED_LAUNCH_SCRIPT], env=dict(os.environ, PYTHONPATH=ROOT), cwd=ROOT, capture_output=True,
+                         text=True, timeout=120)
+    assert res.returncode == 0 and "left at once" in res.stdout, res.stdout[-500:] + res.stderr[-2000:]
