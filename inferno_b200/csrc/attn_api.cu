@@ -146,7 +146,9 @@ const DeviceInfo* device_info() {
     }
     if (state != 2) return nullptr;
     if (entered != dev) {
-        if (!cuda_ok(cudaFree(nullptr))) return nullptr;
+        // a call that makes the context current and, unlike cudaFree(nullptr), is allowed while a stream is being captured
+        cudaFuncAttributes a;
+        if (!cuda_ok(cudaFuncGetAttributes(&a, reinterpret_cast<const void*>(&linear_finish_kernel)))) return nullptr;
         entered = dev;
     }
     return &d;
