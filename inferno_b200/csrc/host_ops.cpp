@@ -15,6 +15,7 @@
 
 #include <ATen/ATen.h>
 #include <ATen/core/LegacyTypeDispatch.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 
@@ -72,10 +73,12 @@ inline void check_status(int rc, const char* where) {
 // The number of entries is bounded by the number of streams a process uses (torch hands out a fixed pool of them).  A call
 // holds its entry's lock while it issues its launches, so two host threads that share a stream cannot interleave the
 // launches of two passes over one scratch buffer.  The table is never destroyed: at process exit the CUDA context may
-// already be gone.
+// already be gone.  Attention and projections have a buffer each: a graph captured with the one must not lose it because an
+// eager call of the other needs more.
 struct Workspace {
     std::mutex launching;
-    Tensor buf;
+    Tensor buf;            // attention; begins with the status header
+    Tensor linear;
 };
 std::mutex g_ws_mutex;
 std::map<std::pair<int, int64_t>, std::unique_ptr<Workspace>>& workspace_table() {
@@ -90,9 +93,16 @@ Workspace& workspace_of(int device, cudaStream_t stream) {
     return *slot;
 }
 // under ws.launching
-void reserve(Workspace& ws, size_t bytes, c10::Device device) {
-    if (!ws.buf.defined() || static_cast<size_t>(ws.buf.numel()) < bytes)
-        ws.buf = at::empty({static_cast<int64_t>(bytes)}, at::TensorOptions().dtype(at::kByte).device(device));
+Tensor empty_bytes(size_t bytes, c10::Device device) { return at::empty({static_cast<int64_t>(bytes)}, at::TensorOptions().dtype(at::kByte).device(device)); }
+void reserve(Tensor& buf, size_t bytes, c10::Device device) {
+    if (!buf.defined() || static_cast<size_t>(buf.numel()) < bytes) buf = empty_bytes(bytes, device);
+}
+// A projection's scratch.  While the stream is being captured it comes from the graph's own memory, and goes back there after the
+// call: the graph then depends on nothing that a later call could replace.
+Tensor linear_scratch(Workspace& ws, size_t bytes, c10::Device device) {
+    if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return empty_bytes(bytes, device);
+    reserve(ws.linear, bytes, device);
+    return ws.linear;
 }
 
 // ---- timing events queued by a harness: one {start, stop} pair per attention call, forward and backward ----------------
@@ -201,7 +211,7 @@ void launch_fwd(const Shape& s, const Operand& q, const Operand& k, const Operan
     cudaStream_t stream = c10::cuda::getCurrentCUDAStream(device.index()).stream();
     Workspace& ws = workspace_of(device.index(), stream);
     std::lock_guard<std::mutex> lock(ws.launching);
-    reserve(ws, bytes, device);
+    reserve(ws.buf, bytes, device);
     TimingScope timing(false);
     if (total_heads > 0) {
         check_status(g_abi.attn_fwd_chunk(q.ptr, k.ptr, v.ptr, o.ptr, lse, &q.lay, &k.lay, &v.lay, &o.lay, total_heads, s.B, s.H, s.T, s.D, scale, causal,
@@ -221,7 +231,7 @@ void launch_bwd(const Shape& s, const Operand& q, const Operand& k, const Operan
     cudaStream_t stream = c10::cuda::getCurrentCUDAStream(device.index()).stream();
     Workspace& ws = workspace_of(device.index(), stream);
     std::lock_guard<std::mutex> lock(ws.launching);
-    reserve(ws, bytes, device);
+    reserve(ws.buf, bytes, device);
     TimingScope timing(true);
     check_status(g_abi.attn_bwd(q.ptr, k.ptr, v.ptr, o.ptr, dO.ptr, lse, dq.ptr, dk.ptr, dv.ptr, &q.lay, &k.lay, &v.lay, &o.lay, &dO.lay, &dq.lay, &dk.lay,
                                 &dv.lay, s.B, s.H, s.T, s.D, scale, causal, s.dtype, math_mode, ws.buf.data_ptr(), ws.buf.numel(),
@@ -444,9 +454,6 @@ void check_bf16_cuda(const Tensor& t, const char* name) {
     TORCH_CHECK_TYPE(t.scalar_type() == at::kBFloat16, "linear: ", name, " must be bfloat16");
 }
 
-// The stream's workspace begins with the attention calls' header (their sticky status); the projections use what follows it.
-constexpr size_t kHeaderBytes = 256;
-
 Tensor linear_forward(const Tensor& x, const Tensor& w, const Tensor& bias) {
     check_linear_shapes(x, w);
     const int64_t K = w.size(0), N = w.size(1);
@@ -469,15 +476,15 @@ Tensor linear_forward(const Tensor& x, const Tensor& w, const Tensor& bias) {
     const size_t bytes = g_abi.linear_workspace_bytes(M, static_cast<int>(K), static_cast<int>(N), IB200_PASS_FWD);
     cudaStream_t stream = c10::cuda::getCurrentCUDAStream(x.device().index()).stream();
     std::unique_lock<std::mutex> lock;
-    void* scratch = nullptr;
+    Tensor scratch;
     if (bytes) {
         Workspace& ws = workspace_of(x.device().index(), stream);
         lock = std::unique_lock<std::mutex>(ws.launching);
-        reserve(ws, kHeaderBytes + bytes, x.device());
-        scratch = static_cast<char*>(ws.buf.data_ptr()) + kHeaderBytes;
+        scratch = linear_scratch(ws, bytes, x.device());
     }
     check_status(g_abi.linear_fwd(x2.data_ptr(), wc.data_ptr(), b.defined() ? b.data_ptr() : nullptr, b.defined() ? dtype_code(b) : IB200_DTYPE_F32,
-                                  y.data_ptr(), M, static_cast<int>(K), static_cast<int>(N), scratch, bytes, reinterpret_cast<ib200_stream_t>(stream)),
+                                  y.data_ptr(), M, static_cast<int>(K), static_cast<int>(N), bytes ? scratch.data_ptr() : nullptr, bytes,
+                                  reinterpret_cast<ib200_stream_t>(stream)),
                  "ib200_linear_fwd_ws");
     return y;
 }
@@ -506,10 +513,10 @@ LinearGrads linear_backward(const Tensor& x, const Tensor& w, const Tensor& dy, 
     cudaStream_t stream = c10::cuda::getCurrentCUDAStream(x.device().index()).stream();
     Workspace& ws = workspace_of(x.device().index(), stream);
     std::lock_guard<std::mutex> lock(ws.launching);
-    reserve(ws, kHeaderBytes + bytes, x.device());
+    const Tensor scratch = linear_scratch(ws, bytes, x.device());
     auto ptr = [](const Tensor& t) -> void* { return t.defined() ? t.data_ptr() : nullptr; };
     check_status(g_abi.linear_bwd(x2.data_ptr(), wc.data_ptr(), dy2.data_ptr(), ptr(g.dx), ptr(g.dw), ptr(g.db), db_bf16 ? IB200_DTYPE_BF16 : IB200_DTYPE_F32, M,
-                                  static_cast<int>(K), static_cast<int>(N), static_cast<char*>(ws.buf.data_ptr()) + kHeaderBytes, bytes,
+                                  static_cast<int>(K), static_cast<int>(N), scratch.data_ptr(), bytes,
                                   reinterpret_cast<ib200_stream_t>(stream)),
                  "ib200_linear_bwd_ws");
     return g;

@@ -51,3 +51,31 @@ def test_the_first_call_of_a_process_or_thread_can_be_captured(what):
     res = subprocess.run([sys.executable, "-c", _FIRST_CALL, what], env=dict(os.environ, PYTHONPATH=ROOT), cwd=ROOT, capture_output=True, text=True,
                          timeout=120)
     assert res.returncode == 0 and "captured and replayed" in res.stdout, res.stdout[-500:] + res.stderr[-2000:]
+
+
+@pytest.mark.parametrize("captured", ["linear", "attention"])
+def test_a_captured_call_keeps_its_scratch_when_a_projection_needs_more(captured):
+    """Replaying a graph after a larger eager projection on the capture stream writes to the graph's own memory, not to what has since been
+    handed to somebody else."""
+    from inferno_b200 import attention as A
+    from inferno_b200.linear import Linear
+    bf16 = lambda *s: torch.randn(*s, device="cuda").to(torch.bfloat16)
+    s = torch.cuda.Stream()
+    with torch.cuda.stream(s):
+        lin, x, dy = Linear(512, 512).cuda().to(torch.bfloat16), bf16(2048, 512).requires_grad_(), bf16(2048, 512)
+        big, xb, dyb = Linear(4096, 4096).cuda().to(torch.bfloat16), bf16(4096, 4096).requires_grad_(), bf16(4096, 4096)
+        q = torch.randn(1, 4, 512, 64, device="cuda")
+        step = (lambda: torch.autograd.grad(lin(x), (x, lin.weight, lin.bias), dy)) if captured == "linear" else (lambda: A.attention_forward(q, q, q))
+        want = [t.clone() for t in step()]
+        s.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            out = step()
+        torch.autograd.grad(big(xb), (xb, big.weight, big.bias), dyb)
+        # whatever that gave back to the allocator is handed out again
+        junk = [torch.full((n,), 7, device="cuda", dtype=torch.uint8) for n in (1 << 16, 1 << 18, 1 << 20, 1 << 21, 1 << 22, 1 << 23) for _ in range(4)]
+        g.replay()
+        s.synchronize()
+        assert all(bool((j == 7).all()) for j in junk)
+        for a, b in zip(out, want):
+            assert float((a.float() - b.float()).norm()) <= 1e-3 * float(b.float().norm())
