@@ -153,7 +153,7 @@ gemm_bf16_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t rank = cluster_ctarank();
     const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
-    AbortCtx ab{abort_flag, prm.status, 0};
+    ResidentAbortCtx ab{abort_flag, prm.status};
 
     if (tid == 0) {
         *abort_flag = 0;
