@@ -504,12 +504,20 @@ int launch_gemms(const GemmDesc* whole, const GemmDesc* other, int split, float*
     if (split == kPartWhole) {
         tiles += p.t[1].tiles;
         pairs = static_cast<int>(tiles < max_pairs ? tiles : max_pairs);
+    } else if (split == kPartReduceBf16) {
+        // Every part is rounded to bf16 as it is added, so a tile is cut into as few equal parts as keep the pairs busy.  Two parts give the same
+        // bits in either order.  (Runs of equal length over all tiles, the rule below, meet in three or four parts of some tiles.)
+        int splits = std::min(8, max_pairs / p.t[1].tiles);
+        while (splits > 1 && p.t[1].k_slices / splits < kMinPartSlices) --splits;
+        pairs = p.t[1].tiles * splits;
+        p.heavy = 0;
+        p.w_heavy = 0;
+        p.w_light = 1;
+        p.w_total = pairs;
     } else {
         // every pair shall end up with the same number of k-slices: `heavy` pairs own one whole tile (k0 slices) more than the rest
         const long long W = static_cast<long long>(p.t[1].tiles) * p.t[1].k_slices, k0 = whole ? p.t[0].k_slices : 0;
-        // partial tiles that are rounded to bf16 as they are added: at most eight per tile
-        const long long min_part = split == kPartReduceBf16 ? std::max<long long>(kMinPartSlices, (p.t[1].k_slices + 6) / 7) : kMinPartSlices;
-        const long long most = std::max(1LL, W / min_part);
+        const long long most = std::max(1LL, W / kMinPartSlices);
         if (p.t[0].tiles < max_pairs) {
             p.heavy = p.t[0].tiles;
             pairs = p.heavy + static_cast<int>(std::min<long long>(max_pairs - p.heavy, most));

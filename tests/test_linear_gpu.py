@@ -101,3 +101,24 @@ def test_bias_may_be_a_slice(offset):
     b = buf[offset:offset + 264]
     y = L.linear_forward(x, w, b)
     assert torch.equal(y, L.linear_forward(x, w, b.clone())) and rel(y, x.float() @ w.float() + b.float()) < 1e-2
+
+
+@pytest.mark.parametrize("M,K,N", [(16384, 768, 2304), (8192, 512, 768), (1000, 768, 768)])
+def test_weight_gradient_without_a_workspace_has_few_roundings(M, K, N):
+    """ib200_linear_bwd adds its parts in bf16.  With tiles of 256 x 256 that leave 74 CTA pairs half idle these have two to eight parts; where
+    two suffice (the first shape: 27 tiles) the result is the same from run to run."""
+    g = torch.Generator(device="cuda").manual_seed(5)
+    x, w, dy = (torch.randn(*s, device="cuda", generator=g).to(torch.bfloat16) for s in ((M, K), (K, N), (M, N)))
+    s = torch.cuda.current_stream().cuda_stream
+    runs = []
+    for _ in range(6):
+        dx, dw, db = torch.empty_like(x), torch.empty_like(w), torch.empty(N, device="cuda")
+        assert _capi.lib().ib200_linear_bwd(x.data_ptr(), w.data_ptr(), dy.data_ptr(), dx.data_ptr(), dw.data_ptr(), db.data_ptr(), M, K, N, s) == _capi.OK
+        runs.append(dw)
+    ref = x.double().t() @ dy.double()
+    parts = min(8, 74 // (-(-K // 256) * -(-N // 256)), M // 64 // 8)
+    # each part and each sum is rounded to 8 bits: relative error of at most 2^-9 of a running sum, whose norm grows as the square root
+    tol = 2.0 ** -9 * (1 + sum(((i + 1) / parts) ** 0.5 for i in range(parts)))
+    assert rel(runs[0].double(), ref) < tol
+    if parts == 2:
+        assert all(torch.equal(r, runs[0]) for r in runs)
