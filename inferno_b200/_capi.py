@@ -107,10 +107,13 @@ def host():
         L = lib()
         if not os.path.isfile(_build.HOST_PATH):
             raise ImportError(f"{_build.HOST_PATH} is missing: build it with `python -m inferno_b200.build` (there is no fallback path)")
-        import torch  # noqa: F401  (the module's shared-library dependencies)
+        import torch      # the module's shared-library dependencies
         spec = importlib.util.spec_from_file_location("_host_ops", _build.HOST_PATH)
         m = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(m)
+        if m.torch_version != torch.__version__.split("+")[0]:
+            raise ImportError(f"{_build.HOST_PATH} was compiled against torch {m.torch_version}, this is {torch.__version__}: "
+                              "build it again with `python -m inferno_b200.build`")
         m.bind(L._name, Ib200Error)
         _host = m
     return _host

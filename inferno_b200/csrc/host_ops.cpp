@@ -12,6 +12,7 @@
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/autograd/saved_variable.h>
+#include <torch/version.h>
 
 #include <ATen/ATen.h>
 #include <ATen/core/LegacyTypeDispatch.h>
@@ -840,4 +841,12 @@ PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_host_ops", nullptr, -1, g_metho
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__host_ops() { return PyModule_Create(&g_module); }
+PyMODINIT_FUNC PyInit__host_ops() {
+    PyObject* m = PyModule_Create(&g_module);
+    // the torch whose classes this module was compiled against
+    if (m && PyModule_AddStringConstant(m, "torch_version", TORCH_VERSION) < 0) {
+        Py_DECREF(m);
+        return nullptr;
+    }
+    return m;
+}

@@ -217,3 +217,13 @@ def test_refusals_with_formatted_messages_raise(built_lib):
             "except RuntimeError as e:\n    assert 'last axis (8)' in str(e)\nelse:\n    raise SystemExit('not refused')\n")
     res = subprocess.run([sys.executable, "-c", code], cwd=ROOT, env=dict(os.environ, PYTHONPATH=ROOT), capture_output=True, text=True, timeout=300)
     assert res.returncode == 0, res.stderr[-2000:]
+
+
+def test_a_host_module_of_another_torch_is_refused(built_lib, monkeypatch):
+    """It shares torch's C++ classes, so it must not be used with a torch whose classes may differ."""
+    import torch
+    assert _capi.host().torch_version == torch.__version__.split("+")[0]
+    monkeypatch.setattr(_capi, "_host", None)
+    monkeypatch.setattr(torch, "__version__", "1.0.0+cu00")
+    with pytest.raises(ImportError, match="compiled against torch"):
+        _capi.host()
