@@ -470,7 +470,7 @@ def run_ours(args, cfg):
     total_flops = cfg.flops()
     value = total_flops / (ms_step * 1e-3) / 1e12
 
-    # Small configurations (a step of a few hundred microseconds, five dependent launches): the same step replayed as one
+    # Small configurations (a step of a few hundred microseconds, four dependent launches): the same step replayed as one
     # CUDA graph, which takes the per-launch gaps out.  Reported beside the stream-launched figure, not instead of it.
     graph = None
     if flush and not args.no_cuda_graph:
@@ -594,8 +594,8 @@ def finish(args, cfg, world, n, T, D, K, W, preload_steps, value, ms_step, fwd_m
         cuda_graph=graph,
         validation=validation,
         e2e=e2e,
-        gpu_launches=(5 if bf16 else 4) * K,
-        kernels_per_step=["prepare_header_kernel", "attn_fwd_persist_kernel", "bwd_prepass_kernel", "attn_bwd_persist_kernel", "dq_finish_kernel"] if bf16 else
+        gpu_launches=4 * K,
+        kernels_per_step=["attn_fwd_persist_kernel", "bwd_prepass_kernel", "attn_bwd_persist_kernel", "dq_finish_kernel"] if bf16 else
                          ["split_bf16_kernel", "attn_fwd_persist_kernel", "bwd_prepass_kernel", "attn_bwd_persist_kernel (adds its dQ partials straight into dQ)"],
         roofline=dict(bound="tensor", kernel=bwd_kernel, achieved=achieved, peak=peak,
                       unit="TFLOP/s", frac=achieved / peak, of=pk["source"] + ("" if bf16 else " sustained bf16 / 3: the split schedule issues three bf16 MMAs per product"),

@@ -53,7 +53,7 @@ enum { IB200_PASS_FWD = 0, IB200_PASS_BWD = 1 };
 
 /* Bytes of device scratch the forward (pass 0) or backward (pass 1) needs for
  * this problem.  The caller owns the allocation; the library never allocates or
- * frees device memory.  The first 256 bytes are a header (device status word, work counter); the
+ * frees device memory.  The first 256 bytes are a header (the device status); the
  * workspace need not be initialised.
  * Replaces nothing one-to-one: the reference's launchers cudaMalloc their own
  * scratch per call (e.g. src/inferno/cuda/cudamaskedfill.cu:86-164). */
@@ -134,7 +134,8 @@ int ib200_linear_bwd(const void* x, const void* w, const void* dy, void* dx, voi
 
 /* The same two calls with scratch from the caller, and a bias (or bias gradient) of either type (IB200_DTYPE_*).  With a
  * workspace a product that is cut along K (few output tiles, long K: the weight gradient) is added up in fp32 and rounded
- * once; without one its parts, at most eight, are rounded to bf16 as they are added.  The workspace need not be
+ * once; without one its parts, at most eight, are rounded to bf16 as they are added.  Either way the parts are added in the
+ * order in which they finish, so that a product of three parts and more can differ from run to run in its last bits.  The workspace need not be
  * initialised; `ib200_linear_workspace_bytes` gives its size (0: none is used; IB200_PASS_BWD always needs one). */
 size_t ib200_linear_workspace_bytes(int M, int K, int N, int pass);
 int ib200_linear_fwd_ws(const void* x, const void* w, const void* bias, int bias_dtype, void* y, int M, int K, int N,

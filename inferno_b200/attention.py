@@ -104,7 +104,7 @@ def queue_timing_events(forward=(), backward=()) -> None:
 
 
 class AttentionBackward:
-    """The differentiable op with every option.  Its backward node (csrc/host_ops.cpp) saves q, k, v, out and lse, produces
+    """The differentiable op with every option, under the name it had as an autograd function.  Its backward node (csrc/host_ops.cpp) saves q, k, v, out and lse, produces
     dq, dk, dv, and plays the role a ``class AttentionBackward : public Node`` would in the reference
     (src/inferno/gradfn/node.h:23-45: ``backward()``, ``release()``, ``get_inputs()``).
     With ``bthd_out`` the output is laid out [B,T,H,D] in memory (returned as a [B,H,T,D] view).  When q, k, v are

@@ -335,7 +335,7 @@ struct BwdLayouts {
     RowLayout q, k, v, o, dO, dq, dk, dv;
 };
 
-// pre-pass (delta, accumulator zeroing, header, fp32 operand splits) -> main kernel -> dQ finish.
+// pre-pass (delta, accumulator zeroing, fp32 operand splits) -> main kernel -> dQ finish.
 // Workspace: [header | dq accumulator | -delta, -lse*log2e | (fp32 only) dense hi/lo bf16 copies of q, k, v, dO].
 template <int D, bool F32>
 int launch_bwd_typed(const void* q, const void* k, const void* v, const void* o, const void* dO, const float* lse,

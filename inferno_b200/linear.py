@@ -3,7 +3,7 @@
 ``Linear::forward`` in the reference is ``matmul(x, W) + b`` with the weight stored ``[in, out]``
 (src/inferno/modules/linear.cpp:19-106); its backward is MMBackward + the bias' sum_to_shape
 (src/inferno/gradfn/mmbackward.cpp:36-98).  Here both directions run on the tcgen05 GEMM of
-``csrc/linear_gemm.cuh`` through the C ABI (bf16 tensors, fp32 bias and accumulation).
+``csrc/linear_gemm.cuh`` through the C ABI (bf16 tensors, a bias of either type, fp32 accumulation).
 """
 from __future__ import annotations
 
@@ -18,12 +18,15 @@ def linear_forward(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None =
 
 
 def linear_backward(x, w, dy, need_dx=True, need_dw=True, need_db=True):
-    """(dx, dw, db) of ``linear_forward``; db is fp32; what is not needed comes back as None."""
+    """(dx, dw, db) of ``linear_forward``; db is fp32; what is not needed comes back as None.
+
+    A dW whose tiles alone would not fill the GPU evenly is cut along the tokens and its parts are added up in fp32 in the order in
+    which they finish: its bits can differ from run to run in the last place.  dx, db and y repeat bit for bit."""
     return _capi.host().linear_backward(x, w, dy, need_dx, need_dw, need_db)
 
 
 class LinearFunction:
-    """The differentiable projection (backward node in csrc/host_ops.cpp)."""
+    """The differentiable projection (backward node in csrc/host_ops.cpp), under the name it had as an autograd function."""
 
     @staticmethod
     def apply(x, w, bias):
